@@ -91,16 +91,12 @@ struct ClassicSeg {
   uint32_t passes;  // coding passes
 };
 
-// 16-bit scratch words a classic block needs: blocks of at most 64 x 64
-// keep four 64-bit planes of rows -1 .. h+3 (69 rows); larger ones one flag
-// word per sample padded by one on every side.  A multiple of 4, so slots
-// stay 8-byte aligned.
+// 16-bit words of shared memory a classic block in flight needs: one per
+// column of each four-row stripe.
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-inline uint32_t classic_slot_words(uint32_t w, uint32_t h) {
-  return (w <= 64 && h <= 64) ? 4u * 69u * 4u : (((w + 2) * (h + 2) + 3) & ~3u);
-}
+constexpr uint32_t classic_slot_words(uint32_t w, uint32_t h) { return w * ((h + 3) / 4); }
 
 // Irreversible (9/7) levels use the same tables: band pointers hold int32
 // coefficients that the kernel dequantises with `step`, level images (the

@@ -534,14 +534,13 @@ sgn_status build_plan_impl(sgn_ctx* ctx, cudaStream_t s, PinnedBuffer& staging, 
   }
   if (cfg.idwt_seg_shift || cfg.pack_seg_shift) set_segments(plan, idwt, packs, cfg.idwt_seg_shift, cfg.pack_seg_shift);
   plan->nclassic = ncls;
-  size_t cscratch_bytes = 0;
   if (ncls) {
     plan->classic_slot = std::max<uint32_t>(cslot, 1);
-    const uint32_t per = classic_threads_per_cta();
-    // As many resident threads as the kernel's occupancy allows (every block
-    // a thread of its own where possible: the slowest block sets the time).
-    plan->classic_ctas = std::min<uint32_t>((ncls + per - 1) / per, (uint32_t)ctx->sm_count * classic_ctas_per_sm());
-    cscratch_bytes = (size_t)plan->classic_ctas * per * plan->classic_slot * sizeof(uint16_t);
+    // Blocks in flight per warp: as few as let every block start at once, up
+    // to what a warp's lanes and its pool of column words hold.
+    const uint32_t slots = (uint32_t)ctx->sm_count * classic_ctas_per_sm();
+    plan->classic_lanes = std::min((ncls + slots - 1) / slots, classic_max_lanes(plan->classic_slot));
+    plan->classic_ctas = std::min((ncls + plan->classic_lanes - 1) / plan->classic_lanes, slots);
   }
   plan->nqueues = (uint32_t)plan->rounds.size() + 3 + kPackVariants;
 
@@ -558,9 +557,9 @@ sgn_status build_plan_impl(sgn_ctx* ctx, cudaStream_t s, PinnedBuffer& staging, 
   if ((e = staging.ensure(stage_bytes)) != cudaSuccess) return cuda_status(e, "pinned staging");
   {
     // One table arena: the job tables in their staging layout (uploaded by
-    // one copy), then the work-queue counters and the classic scratch.
-    const size_t tab = stage_bytes - at_ht, at_q = up16(tab), at_cs = at_q + up16((size_t)plan->nqueues * 4);
-    if ((e = cudaMallocAsync(&plan->d_tables, at_cs + std::max<size_t>(cscratch_bytes, 16), s)) != cudaSuccess)
+    // one copy), then the work-queue counters.
+    const size_t at_q = up16(stage_bytes - at_ht);
+    if ((e = cudaMallocAsync(&plan->d_tables, at_q + up16((size_t)plan->nqueues * 4), s)) != cudaSuccess)
       return cuda_status(e, "table arena");
     uint8_t* base = static_cast<uint8_t*>(plan->d_tables);
     plan->d_ht = nht ? reinterpret_cast<HtJob*>(base) : nullptr;
@@ -571,7 +570,6 @@ sgn_status build_plan_impl(sgn_ctx* ctx, cudaStream_t s, PinnedBuffer& staging, 
     plan->d_csegs = ncls ? reinterpret_cast<ClassicSeg*>(base + (at_cseg - at_ht)) : nullptr;
     plan->d_gather = gather_total ? base + (at_gather - at_ht) : nullptr;
     plan->d_queue = reinterpret_cast<uint32_t*>(base + at_q);
-    plan->d_cscratch = cscratch_bytes ? reinterpret_cast<uint16_t*>(base + at_cs) : nullptr;
   }
   uint8_t* st = staging.p;
   HtJob* ht = reinterpret_cast<HtJob*>(st + at_ht);
@@ -766,8 +764,8 @@ sgn_status apply_config(sgn_ctx* ctx, sgn_plan* p, const LaunchConfig& in) {
 }
 
 cudaError_t launch_classic_blocks(const sgn_plan* p, cudaStream_t s) {
-  return launch_classic(p->d_classic, p->d_csegs, p->nclassic, p->d_input, p->d_gather, p->d_coef, p->d_cscratch,
-                        p->classic_slot, p->classic_ctas, p->d_queue + p->rounds.size() + 2 + kPackVariants, s);
+  return launch_classic(p->d_classic, p->d_csegs, p->nclassic, p->d_input, p->d_gather, p->d_coef, p->classic_slot,
+                        p->classic_ctas, p->classic_lanes, p->d_queue + p->rounds.size() + 2 + kPackVariants, s);
 }
 
 cudaError_t launch_round(const sgn_plan* p, size_t k, cudaStream_t s, bool queued, uint32_t ctas, bool lean) {
@@ -807,7 +805,6 @@ void free_plan_buffers(sgn_plan* p, cudaStream_t s) {
   p->d_refine = nullptr;
   p->d_classic = nullptr;
   p->d_csegs = nullptr;
-  p->d_cscratch = nullptr;
   p->d_gather = nullptr;
   p->d_idwt = nullptr;
   p->d_pack = nullptr;

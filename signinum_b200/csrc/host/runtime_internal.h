@@ -182,7 +182,7 @@ struct sgn_plan {
   // Device allocations (stream-ordered pool): the input arena, and two
   // arenas the buffers below are parts of: d_work (coefficients, level
   // planes, quad symbols, tile status) and d_tables (job tables, work-queue
-  // counters, classic scratch).
+  // counters).
   void* d_work = nullptr;
   void* d_tables = nullptr;
   uint8_t* d_input = nullptr;
@@ -192,12 +192,11 @@ struct sgn_plan {
   uint32_t* d_symbols = nullptr;
   HtJob* d_ht = nullptr;
   uint32_t* d_refine = nullptr;
-  // Classic (EBCOT) code blocks: jobs, segment table, per-thread flag scratch.
+  // Classic (EBCOT) code blocks: jobs, segment table.
   ClassicJob* d_classic = nullptr;
   ClassicSeg* d_csegs = nullptr;
-  uint16_t* d_cscratch = nullptr;
   uint8_t* d_gather = nullptr;  // multi-layer classic blocks' data, gathered per block
-  uint32_t nclassic = 0, classic_ctas = 0, classic_slot = 0;
+  uint32_t nclassic = 0, classic_ctas = 0, classic_lanes = 0, classic_slot = 0;
   IdwtJob* d_idwt = nullptr;
   PackJob* d_pack = nullptr;
   uint32_t* d_status = nullptr;

@@ -10,15 +10,33 @@
 // (sign x magnitude, bit 0 the least significant decoded bit-plane), the
 // layout the HT kernels write, so the IDWT and pack kernels run unchanged.
 //
-// Mapping: the MQ decoder is one serial chain per code block, so a thread
-// decodes a block.  A persistent grid of threads takes blocks from a device
-// counter.  Each thread owns a slot of 16-bit flag words in global scratch,
-// one per sample of the block padded by one on every side (low byte: the
-// significance of the eight neighbours, as the reference keeps it; high
-// byte: significant, refined, coded in this bit-plane, sign); the magnitude
-// bits accumulate in place in the coefficient arena.  The probability table,
-// the context-label tables and each thread's 19 context states live in
-// shared memory.
+// Mapping: the MQ decoder is one serial chain per code block, so a lane
+// decodes a block, `lanes` of them per warp, each taking blocks from a device
+// counter.  The lanes of a warp are at different places of different blocks,
+// so the decoder is one loop that every lane runs in step: an iteration steps
+// to the next column when the current one is done, picks the next sample that
+// the pass codes, decodes one binary decision (zero coding, sign, refinement,
+// run length or uniform, whichever the lane's position asks for) through the
+// one copy of the MQ decoder, and applies its bit.  Rare events (stripe, pass
+// and block ends, raw segments) are branches; the rest is straight-line code
+// under selects, whose independent parts (column step, probability update,
+// renormalisation) overlap.
+//
+// A stripe column's state is one 16-bit word in shared memory (significance,
+// sign, refined and coded flags of its four samples).  A column and its two
+// neighbours, each joined with the samples above and below the stripe, hold
+// the whole context window; they sit in registers while the column is coded,
+// and the next column's words are loaded one column ahead.
+//
+// What bounds it: the chain of decisions of the plan's longest block (some
+// 40,000 of them in a 64 x 64 block of noise), every decision a fixed-latency
+// path of table loads and selects in a warp that has its scheduler almost to
+// itself.  64 tiles of 512 x 512 RGB (13,440 blocks): 41.6 ms with a thread
+// per block and nested pass loops, whose 32 lanes took turns at their
+// branches (10.5 M warp instructions per warp), 21.1 ms in this form with 16
+// blocks per warp; one tile (210 blocks, one per warp) 13.7 ms, with all of
+// them in seven warps 18.3 ms.  The same loop with a branch per kind of
+// decision took 27 ms (24 ms for one tile with 16 blocks per warp).
 #include <algorithm>
 #include <cstdint>
 
@@ -31,479 +49,160 @@ namespace {
 
 using namespace ebcot;
 
-constexpr int kClassicThreads = 128;
-constexpr uint16_t kSigF = 0x8000, kRefF = 0x4000, kCodF = 0x2000, kSgnF = 0x1000;
+// One warp per CTA in the launches below; at most 32 blocks in flight per
+// CTA, whose column words share one pool (16 blocks of 64 x 64).
+constexpr uint32_t kClassicThreads = 32, kClassicBlocks = 32;
+constexpr uint32_t kClassicPool = 16 * classic_slot_words(64, 64);
 
+// Column word in shared memory: bits 0..3 significant, 4..7 refined, 8..11
+// sign, 12..15 coded in this bit-plane (rows 0 .. 3 of the stripe).  In
+// registers, joined with the rows above and below (join): bits 0..5
+// significance of rows -1 .. 4, bits 8..13 their signs, 16..19 refined,
+// 24..27 coded.
+constexpr int kSgnBit = 8, kRefBit = 16, kCodBit = 24;
+constexpr uint32_t kCodMask = 0xFu << kCodBit;
+
+__device__ __forceinline__ uint32_t join(uint32_t above, uint32_t own, uint32_t below) {
+  return ((own & 0x0F0Fu) << 1) | ((own & 0xF0F0u) << 12) | ((above >> 3) & 0x0101u) | ((below & 0x0101u) << 5);
+}
+__device__ __forceinline__ uint16_t own_word(uint32_t c) {
+  return (uint16_t)(((c >> 1) & 0x0F0Fu) | ((c >> 12) & 0xF0F0u));
+}
+
+// The 3 x 3 significance window of row k from the columns' significance
+// bits Q (left | centre << 9 | right << 18, rows -1 .. 4 from bit 0): the
+// three rows k-1 .. k+1 of the left column in bits 0..2, of the centre in
+// 3..5 (the sample itself bit 4), of the right in 6..8.
+__device__ __forceinline__ uint32_t zc_index(uint32_t Q, uint32_t k) {
+  const uint32_t t = (Q >> k) & 0x1C0E07u;
+  return (t | (t >> 6) | (t >> 12)) & 0x1FFu;
+}
+constexpr uint32_t kCentre = 1u << 4;
+
+// The neighbour-significance byte of ebcot.h for a window index.
+__device__ __forceinline__ uint8_t window_byte(uint32_t i) {
+  return (uint8_t)(((i & 1) << 7) | (((i >> 3) & 1) << 6) | (((i >> 6) & 1) << 5) | (((i >> 1) & 1) << 4) |
+                   (((i >> 2) & 1) << 3) | (((i >> 7) & 1) << 2) | (((i >> 8) & 1) << 1) | ((i >> 5) & 1));
+}
+
+// Significance (bits 0..3) and signs (bits 4..7) of the left, right, upper
+// and lower neighbours of row k from the column words.
+__device__ __forceinline__ uint32_t sign_index(uint32_t L, uint32_t C, uint32_t R, uint32_t k) {
+  const uint32_t l = (L >> (k + 1)) & 0x101u, r = (R >> (k + 1)) & 0x101u, c = C >> k;
+  const uint32_t v = l | (r << 1) | ((c & 0x101u) << 2) | (((c >> 2) & 0x101u) << 3);
+  return (v | (v >> 4)) & 0xFFu;
+}
+// Its byte of sc_context: two bits (negative, positive) per neighbour, top,
+// left, right, bottom from the high end.
+__device__ __forceinline__ uint8_t sign_byte(uint32_t i) {
+  uint32_t m = 0;
+  const uint32_t place[4] = {4, 2, 6, 0};  // left, right, upper, lower
+  for (int n = 0; n < 4; ++n)
+    if ((i >> n) & 1) m |= 1u << (place[n] + ((i >> (4 + n)) & 1));
+  return (uint8_t)m;
+}
+
+// A context's adaptive state is its word of the probability table (Table
+// C.2) for (index, MPS): qe, bits 16..22 the entry after an MPS, 23..29 the
+// entry after an LPS (the MPS switched where the table says so), bit 31 the
+// MPS; entry 2 * index + MPS.
 struct Tables {
-  uint32_t qe[47];  // qe | nmps << 16 | nlps << 23 | switch << 30
-  uint8_t zc[3][256];
-  uint8_t sc[256];  // label | xor << 7
-  uint8_t cx[19][kClassicThreads];  // per thread: index | mps << 7
+  uint32_t state[94];
+  uint8_t zc[3][512];  // zero-coding label by window index (zc_index)
+  uint8_t sc[256];     // sign label | xor << 7 by sign index (sign_index)
+  uint32_t cx[19][kClassicBlocks];
+  uint16_t cols[kClassicPool];
 };
 
+// The MQ decoder of Annex C (C in the inverted form of the reference).  The
+// current byte and the one after it are held, so that a refill never waits
+// for the byte it appends.
 struct MqDec {
   const uint8_t* d;
-  uint32_t len, bp, c, a, ct;
+  uint32_t len, bp, b0, b1, c, a, ct;
   __device__ __forceinline__ uint32_t byte_at(uint32_t i) const { return i < len ? (uint32_t)__ldg(d + i) : 0xFFu; }
   __device__ __forceinline__ void bytein() {
-    if (byte_at(bp) == 0xFF) {
-      if (byte_at(bp + 1) > 0x8F) {
-        ct = 8;
-      } else {
-        ++bp;
-        c = c + 0xFE00u - (byte_at(bp) << 9);
-        ct = 7;
-      }
-    } else {
+    const uint32_t stuffed = b0 == 0xFF ? 1u : 0u;
+    const bool end = stuffed && b1 > 0x8F;  // a marker: zeros (ones in the reference's form) from here on
+    c += end ? 0u : 0xFF00u - (stuffed << 8) - (b1 << (8 + stuffed));
+    ct = end ? 8 : 8 - stuffed;
+    if (!end) {
       ++bp;
-      c = c + 0xFF00u - (byte_at(bp) << 8);
-      ct = 8;
+      b0 = b1;
+      b1 = byte_at(bp + 1);
     }
   }
   __device__ __forceinline__ void init(const uint8_t* data, uint32_t n) {
     d = data;
     len = n;
     bp = 0;
-    c = (byte_at(0) ^ 0xFFu) << 16;
+    b0 = byte_at(0);
+    b1 = byte_at(1);
+    c = (b0 ^ 0xFFu) << 16;
     bytein();
     c <<= 7;
     ct -= 7;
     a = 0x8000;
   }
-  __device__ __forceinline__ uint32_t decode(uint8_t& cx, const uint32_t* qe) {
-    const uint32_t e = qe[cx & 0x7F];
-    const uint32_t q = e & 0xFFFF, mps = cx >> 7;
-    a -= q;
-    uint32_t dbit;
-    if ((c >> 16) < a) {
-      if (a & 0x8000) return mps;
-      if (a < q) {  // MPS exchange
-        dbit = 1 - mps;
-        cx = (uint8_t)((((e >> 23) & 0x7F)) | ((mps ^ ((e >> 30) & 1)) << 7));
-      } else {
-        dbit = mps;
-        cx = (uint8_t)(((e >> 16) & 0x7F) | (mps << 7));
-      }
-    } else {
-      c -= a << 16;
-      if (a < q) {  // LPS exchange
-        a = q;
-        dbit = mps;
-        cx = (uint8_t)(((e >> 16) & 0x7F) | (mps << 7));
-      } else {
-        a = q;
-        dbit = 1 - mps;
-        cx = (uint8_t)(((e >> 23) & 0x7F) | ((mps ^ ((e >> 30) & 1)) << 7));
-      }
+  // One decision with a context whose state is e; an e of 0 changes nothing
+  // and gives 0.  *cx receives the context's next state.
+  __device__ __forceinline__ uint32_t decode(uint32_t e, uint32_t* cx, const uint32_t* state) {
+    const uint32_t q = e & 0xFFFFu, rest = a - q;
+    const bool low = (c >> 16) >= rest;   // the LPS sub-interval
+    const bool lps = low != (rest < q);   // with the conditional exchange
+    c -= low ? rest << 16 : 0u;
+    a = low ? q : rest;
+    // RENORMD (C.3.3), as many bits at once as A needs and the byte buffer
+    // holds (as the reference's renormalize does); a decision seldom needs
+    // more than one byte.
+    uint32_t sh = (uint32_t)__clz(a) - 16;
+    if (sh) *cx = state[(e >> (lps ? 23 : 16)) & 0x7Fu];
+    a <<= sh;
+    uint32_t s1 = min(sh, ct);
+    c <<= s1;
+    ct -= s1;
+    sh -= s1;
+    if (sh) bytein();
+    s1 = min(sh, ct);
+    c <<= s1;
+    ct -= s1;
+    sh -= s1;
+    while (sh) {
+      bytein();
+      s1 = min(sh, ct);
+      c <<= s1;
+      ct -= s1;
+      sh -= s1;
     }
-    // RENORMD (C.3.3), shifting as many bits at once as A needs and the
-    // byte buffer holds (as the reference's renormalize does).
-    while ((a & 0x8000) == 0) {
-      if (ct == 0) bytein();
-      const uint32_t sh = min((uint32_t)__clz(a) - 16, ct);
-      a <<= sh;
-      c <<= sh;
-      ct -= sh;
-    }
-    return dbit;
+    return (e >> 31) ^ (lps ? 1u : 0u);
+  }
+  // A bypassed segment: d, len, and bp as a bit position.
+  __device__ __forceinline__ void init_raw(const uint8_t* data, uint32_t n) {
+    d = data;
+    len = n;
+    bp = 0;
   }
 };
 
-// Raw bits of a bypassed segment: packet-header stuffing; 1 past the end or on
-// a bad stuff bit (the reference's non-strict BypassDecoder).
-struct RawDec {
-  const uint8_t* d;
-  uint32_t len, cur;
-  __device__ __forceinline__ bool bit(uint32_t& b) {
-    if ((cur >> 3) >= len) return false;
-    b = (__ldg(d + (cur >> 3)) >> (7 - (cur & 7))) & 1;
-    ++cur;
-    return true;
+// The raw bit at position p of a bypassed segment (bit 0 of the result, the
+// next position above it): packet-header stuffing; 1 past the end or on a bad
+// stuff bit (the reference's non-strict BypassDecoder).
+__device__ __noinline__ uint32_t raw_bit(const uint8_t* d, uint32_t len, uint32_t p) {
+  if ((p >> 3) >= len) return (p << 1) | 1u;
+  const uint32_t byte = __ldg(d + (p >> 3));
+  uint32_t b = (byte >> (7 - (p & 7))) & 1u;
+  const bool stuff = (p & 7) == 7 && byte == 0xFF;
+  ++p;
+  if (stuff) {
+    if ((p >> 3) >= len) return (p << 1) | 1u;
+    b |= (__ldg(d + (p >> 3)) >> (7 - (p & 7))) & 1u;
+    ++p;
   }
-  __device__ __forceinline__ uint32_t decode(uint8_t&, const uint32_t*) {
-    const bool stuff = (cur & 7) == 7 && (cur >> 3) < len && __ldg(d + (cur >> 3)) == 0xFF;
-    uint32_t b;
-    if (!bit(b)) return 1;
-    if (stuff) {
-      uint32_t s;
-      if (!bit(s) || s != 0) return 1;
-    }
-    return b;
-  }
-};
-
-struct Block {
-  uint16_t* f;    // flag words, (w + 2) x (h + 2)
-  uint32_t* out;  // coefficients, row stride `stride`
-  uint32_t w, h, pw, stride, pos;
-  uint8_t band, style;
-  Tables* t;
-  int tid;
-  __device__ __forceinline__ uint8_t& cx(int label) { return t->cx[label][tid]; }
-  __device__ __forceinline__ uint32_t fi(uint32_t x, uint32_t y) const { return (y + 1) * pw + x + 1; }
-  __device__ __forceinline__ uint32_t& co(uint32_t x, uint32_t y) { return out[(size_t)y * stride + x]; }
-  __device__ __forceinline__ bool next_stripe(uint32_t y) const { return y + 1 < h && ((y + 1) >> 2) > (y >> 2); }
-  __device__ __forceinline__ uint8_t nbr(uint32_t i, uint32_t y) const {
-    const uint8_t n = (uint8_t)f[i];
-    return ((style & kVCausal) && next_stripe(y)) ? (uint8_t)(n & 0xF4) : n;
-  }
-  __device__ __forceinline__ void set_significant(uint32_t i) {
-    f[i] |= kSigF;
-    f[i - pw - 1] |= 1 << 1;
-    f[i - pw] |= 1 << 0;
-    f[i - pw + 1] |= 1 << 3;
-    f[i - 1] |= 1 << 2;
-    f[i + 1] |= 1 << 4;
-    f[i + pw - 1] |= 1 << 5;
-    f[i + pw] |= 1 << 6;
-    f[i + pw + 1] |= 1 << 7;
-  }
-  __device__ __forceinline__ uint32_t sgn(uint32_t i) const { return (f[i] >> 12) & 1; }
-  template <typename D>
-  __device__ __forceinline__ void decode_sign(uint32_t i, uint32_t x, uint32_t y, D& dec, bool raw) {
-    const uint8_t s = nbr(i, y) & 0x55;
-    const uint32_t bottom = ((style & kVCausal) && next_stripe(y)) ? 0 : sgn(i + pw);
-    const uint32_t signs = (sgn(i - pw) << 6) | (sgn(i - 1) << 4) | (sgn(i + 1) << 2) | bottom;
-    const uint8_t e = t->sc[(uint8_t)(((s & signs) << 1) | (s & ~signs))];
-    uint32_t b = dec.decode(cx(e & 0x7F), t->qe);
-    if (!raw) b ^= e >> 7;
-    if (b) {
-      f[i] |= kSgnF;
-      co(x, y) |= 0x80000000u;
-    }
-  }
-  template <typename D>
-  __device__ __forceinline__ void cleanup_one(uint32_t x, uint32_t y, D& dec, bool raw) {
-    const uint32_t i = fi(x, y);
-    if (f[i] & (kSigF | kCodF)) return;
-    const uint32_t b = dec.decode(cx(t->zc[band][nbr(i, y)]), t->qe);
-    if (b) {
-      co(x, y) |= 1u << pos;
-      decode_sign(i, x, y, dec, raw);
-      set_significant(i);
-    }
-  }
-  template <typename D>
-  __device__ void cleanup(D& dec, bool raw) {
-    for (uint32_t by = 0; by < h; by += 4) {
-      const uint32_t ye = min(by + 4, h);
-      for (uint32_t x = 0; x < w; ++x) {
-        bool run = ye - by == 4;
-        for (uint32_t y = by; run && y < ye; ++y) {
-          const uint32_t i = fi(x, y);
-          run = !(f[i] & (kSigF | kCodF)) && nbr(i, y) == 0;
-        }
-        if (run) {
-          if (dec.decode(cx(17), t->qe) == 0) continue;
-          uint32_t k = dec.decode(cx(18), t->qe) << 1;
-          k |= dec.decode(cx(18), t->qe);
-          const uint32_t sy = by + k, i = fi(x, sy);
-          co(x, sy) |= 1u << pos;
-          decode_sign(i, x, sy, dec, raw);
-          set_significant(i);
-          for (uint32_t y = sy + 1; y < ye; ++y) cleanup_one(x, y, dec, raw);
-          continue;
-        }
-        for (uint32_t y = by; y < ye; ++y) cleanup_one(x, y, dec, raw);
-      }
-    }
-  }
-  template <typename D>
-  __device__ void sig_prop(D& dec, bool raw) {
-    for (uint32_t by = 0; by < h; by += 4) {
-      const uint32_t ye = min(by + 4, h);
-      for (uint32_t x = 0; x < w; ++x)
-        for (uint32_t y = by; y < ye; ++y) {
-          const uint32_t i = fi(x, y);
-          const uint8_t n = nbr(i, y);
-          if ((f[i] & kSigF) || n == 0) continue;
-          const uint32_t b = dec.decode(cx(t->zc[band][n]), t->qe);
-          f[i] |= kCodF;
-          if (b) {
-            co(x, y) |= 1u << pos;
-            decode_sign(i, x, y, dec, raw);
-            set_significant(i);
-          }
-        }
-    }
-  }
-  template <typename D>
-  __device__ void mag_ref(D& dec) {
-    for (uint32_t by = 0; by < h; by += 4) {
-      const uint32_t ye = min(by + 4, h);
-      for (uint32_t x = 0; x < w; ++x)
-        for (uint32_t y = by; y < ye; ++y) {
-          const uint32_t i = fi(x, y);
-          const uint16_t fl = f[i];
-          if (!(fl & kSigF) || (fl & kCodF)) continue;
-          const uint32_t b = dec.decode(cx(mr_context((fl & kRefF) != 0, nbr(i, y))), t->qe);
-          co(x, y) |= b << pos;
-          f[i] |= kRefF;
-        }
-    }
-  }
-  __device__ void reset_contexts() {
-    for (int k = 0; k < 19; ++k) cx(k) = initial_index(k);
-  }
-  template <typename D>
-  __device__ void passes(uint32_t start, uint32_t end, uint32_t bitplanes, D& dec, bool raw) {
-    for (uint32_t p = start; p < end; ++p) {
-      pos = bitplanes - 1 - (p + 2) / 3;
-      const uint32_t kind = p % 3;
-      if (kind == 0) {
-        cleanup(dec, raw);
-        if (style & kSegSym)
-          for (int k = 0; k < 4; ++k) dec.decode(cx(18), t->qe);
-        for (uint32_t y = 0; y < h; ++y)
-          for (uint32_t x = 0; x < w; ++x) f[fi(x, y)] &= (uint16_t)~kCodF;
-      } else if (kind == 1) {
-        sig_prop(dec, raw);
-      } else {
-        mag_ref(dec);
-      }
-      if (style & kReset) reset_contexts();
-    }
-  }
-};
-
-// Blocks of at most 64 x 64 samples: per row four 64-bit planes (bit x =
-// column x) in the thread's scratch slot, rows -1 .. h+3 with zero padding:
-// significant, sign, refined, coded in this bit-plane.  A pass walks the
-// stripes; the six rows around a stripe live in registers while its columns
-// are scanned (the neighbour-significance byte of a sample is assembled from
-// three-bit windows of the rows above, at and below it), and the four rows
-// of the stripe go back at its end.  Magnitude and sign bits are OR-ed into
-// the coefficient words with reductions that nothing waits on.
-constexpr uint32_t kSmallRows = 64 + 5;
-static_assert(4 * kSmallRows * 4 == 1104, "small-block slot of classic_slot_words");
-
-struct Small {
-  uint64_t* P;  // sig, sgn, ref, cod planes of kSmallRows rows; row y at y + 1
-  uint32_t* out;
-  uint32_t w, h, stride, pos;
-  uint8_t band, style;
-  Tables* t;
-  int tid;
-  __device__ __forceinline__ uint8_t& cx(int label) { return t->cx[label][tid]; }
-  __device__ __forceinline__ uint64_t* plane(int k) { return P + k * kSmallRows; }
-  // Bits x-1, x, x+1 of a row (columns outside the block read 0).
-  __device__ static __forceinline__ uint32_t w3(uint64_t r, uint32_t x) {
-    return (uint32_t)(x ? (r >> (x - 1)) : (r << 1)) & 7u;
-  }
-  __device__ static __forceinline__ uint32_t bit_at(uint64_t r, uint32_t x) { return (uint32_t)(r >> x) & 1u; }
-  __device__ __forceinline__ void reset_contexts() {
-    for (int k = 0; k < 19; ++k) cx(k) = initial_index(k);
-  }
-
-  template <int KIND, typename D>
-  __device__ void pass(D& dec, bool raw) {
-    uint64_t* S = plane(0);
-    uint64_t* G = plane(1);
-    uint64_t* R = plane(2);
-    uint64_t* C = plane(3);
-    const bool vcausal = style & kVCausal;
-    for (uint32_t y0 = 0; y0 < h; y0 += 4) {
-      const uint32_t nr = min(4u, h - y0);
-      uint64_t s[6], g[6], c[4], r[4];
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        s[k] = S[y0 + k];
-        g[k] = G[y0 + k];
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        c[k] = C[y0 + 1 + k];
-        r[k] = R[y0 + 1 + k];
-      }
-      // Vertically causal: the stripe's last row ignores the row below it.
-      const bool cut = vcausal && y0 + 4 < h;
-      for (uint32_t x = 0; x < w; ++x) {
-        const uint64_t bx = 1ull << x;
-        auto nbr = [&](int k) -> uint32_t {
-          const uint32_t u = w3(s[k], x), m = w3(s[k + 1], x), d = (cut && k == 3) ? 0u : w3(s[k + 2], x);
-          return ((u & 1) << 7) | ((u & 2) << 5) | ((u & 4) << 3) | ((m & 1) << 4) | ((d & 1) << 3) | (m & 4) |
-                 ((d & 4) >> 1) | ((d & 2) >> 1);
-        };
-        auto sign = [&](int k, uint32_t n) {
-          const uint32_t sg = n & 0x55;
-          const uint32_t top = bit_at(g[k], x), left = x ? bit_at(g[k + 1], x - 1) : 0u;
-          const uint32_t right = x < 63 ? bit_at(g[k + 1], x + 1) : 0u;
-          const uint32_t bottom = (cut && k == 3) ? 0u : bit_at(g[k + 2], x);
-          const uint32_t signs = (top << 6) | (left << 4) | (right << 2) | bottom;
-          const uint8_t e = t->sc[(uint8_t)(((sg & signs) << 1) | (sg & ~signs))];
-          uint32_t b = dec.decode(cx(e & 0x7F), t->qe);
-          if (!raw) b ^= e >> 7;
-          return b;
-        };
-        uint32_t* col = out + (size_t)y0 * stride + x;
-        // A sample turning significant: its magnitude bit, sign, and state.
-        auto significant = [&](int k, uint32_t n) {
-          const uint32_t sb = sign(k, n);
-          atomicOr(col + (size_t)k * stride, (1u << pos) | (sb << 31));
-          s[k + 1] |= bx;
-          if (sb) g[k + 1] |= bx;
-        };
-        if (KIND == 0) {
-          int first = 0;
-          if (nr == 4) {
-            bool run = true;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) run = run && !((s[k + 1] | c[k]) & bx) && nbr(k) == 0;
-            if (run) {
-              if (dec.decode(cx(17), t->qe) == 0) continue;
-              uint32_t f = dec.decode(cx(18), t->qe) << 1;
-              f |= dec.decode(cx(18), t->qe);
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                if ((uint32_t)k == f) significant(k, nbr(k));
-              first = (int)f + 1;
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (k < first || (uint32_t)k >= nr || ((s[k + 1] | c[k]) & bx)) continue;
-            const uint32_t n = nbr(k);
-            if (dec.decode(cx(t->zc[band][n]), t->qe)) significant(k, n);
-          }
-        } else if (KIND == 1) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if ((uint32_t)k >= nr || (s[k + 1] & bx)) continue;
-            const uint32_t n = nbr(k);
-            if (n == 0) continue;
-            c[k] |= bx;
-            if (dec.decode(cx(t->zc[band][n]), t->qe)) significant(k, n);
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if ((uint32_t)k >= nr || !(s[k + 1] & bx) || (c[k] & bx)) continue;
-            const uint32_t b = dec.decode(cx(mr_context((r[k] & bx) != 0, nbr(k))), t->qe);
-            if (b) atomicOr(col + (size_t)k * stride, 1u << pos);
-            r[k] |= bx;
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if ((uint32_t)k >= nr) continue;
-        S[y0 + 1 + k] = s[k + 1];
-        G[y0 + 1 + k] = g[k + 1];
-        R[y0 + 1 + k] = r[k];
-        C[y0 + 1 + k] = KIND == 0 ? 0ull : c[k];  // the cleanup pass ends the bit-plane
-      }
-    }
-  }
-
-  template <typename D>
-  __device__ void passes(uint32_t start, uint32_t end, uint32_t bitplanes, D& dec, bool raw) {
-    for (uint32_t p = start; p < end; ++p) {
-      pos = bitplanes - 1 - (p + 2) / 3;
-      const uint32_t kind = p % 3;
-      if (kind == 0) {
-        pass<0>(dec, raw);
-        if (style & kSegSym)
-          for (int k = 0; k < 4; ++k) dec.decode(cx(18), t->qe);
-      } else if (kind == 1) {
-        pass<1>(dec, raw);
-      } else {
-        pass<2>(dec, raw);
-      }
-      if (style & kReset) reset_contexts();
-    }
-  }
-};
-
-__device__ void decode_general(const ClassicJob& job, const ClassicSeg* __restrict__ segs, const uint8_t* data,
-                               uint32_t* out, uint16_t* slot, Tables* t);
-
-template <typename B>
-__device__ __forceinline__ void run_passes(B& b, const ClassicJob& job, const ClassicSeg* __restrict__ segs,
-                                           const uint8_t* data) {
-  const uint32_t max_passes = 1 + 3 * ((uint32_t)job.bitplanes - 1);
-  if (!(job.style & (kBypass | kTermAll))) {
-    uint32_t total = 0;
-    for (uint32_t k = 0; k < job.nseg; ++k) total += segs[job.seg + k].len;
-    MqDec dec;
-    dec.init(data, total);
-    b.passes(0, min((uint32_t)job.passes, max_passes), job.bitplanes, dec, false);
-    return;
-  }
-  uint32_t start = 0, off = 0;
-  for (uint32_t k = 0; k < job.nseg; ++k) {
-    const ClassicSeg s = segs[job.seg + k];
-    const uint32_t end = min(start + s.passes, max_passes);
-    if (segment_is_arithmetic(job.style, start)) {
-      MqDec dec;
-      dec.init(data + off, s.len);
-      b.passes(start, end, job.bitplanes, dec, false);
-    } else {
-      RawDec dec{data + off, s.len, 0};
-      b.passes(start, end, job.bitplanes, dec, true);
-    }
-    start += s.passes;
-    off += s.len;
-  }
+  return (p << 1) | b;
 }
 
-__device__ void decode_block(const ClassicJob& job, const ClassicSeg* __restrict__ segs,
-                             const uint8_t* __restrict__ input, const uint8_t* __restrict__ gather,
-                             int32_t* __restrict__ coef, uint16_t* slot, Tables* t) {
-  const uint32_t w = job.w, h = job.h, stride = job.stride;
-  // The block's segments, in the input or (multi-layer) in the gather area.
-  const uint8_t* data =
-      (job.src & kClassicGathered) ? gather + (job.src & ~kClassicGathered) : input + job.src;
-  uint32_t* out = reinterpret_cast<uint32_t*>(coef + job.dst);
-  for (uint32_t y = 0; y < h; ++y)
-    for (uint32_t x = 0; x < w; ++x) out[(size_t)y * stride + x] = 0;
-  if (job.passes == 0 || job.bitplanes == 0) return;
-  if (w <= 64 && h <= 64) {
-    Small b;
-    b.P = reinterpret_cast<uint64_t*>(slot);
-    b.out = out;
-    b.w = w;
-    b.h = h;
-    b.stride = stride;
-    b.pos = 0;
-    b.band = job.band_class;
-    b.style = job.style;
-    b.t = t;
-    b.tid = threadIdx.x;
-    for (uint32_t i = 0; i < 4 * kSmallRows; ++i) b.P[i] = 0;
-    b.reset_contexts();
-    run_passes(b, job, segs, data);
-  } else {
-    decode_general(job, segs, data, out, slot, t);
-  }
-  // The magnitude and sign bits arrived by reductions in L2: read them there.
-  for (uint32_t y = 0; y < h; ++y)
-    for (uint32_t x = 0; x < w; ++x) {
-      const uint32_t v = __ldcg(out + (size_t)y * stride + x);
-      const int32_t m = (int32_t)(v & 0x7FFFFFFFu);
-      out[(size_t)y * stride + x] = (uint32_t)((v >> 31) ? -m : m);
-    }
-}
-
-// Blocks wider or taller than 64: one 16-bit flag word per padded sample.
-__device__ void decode_general(const ClassicJob& job, const ClassicSeg* __restrict__ segs, const uint8_t* data,
-                               uint32_t* out, uint16_t* slot, Tables* t) {
-  const uint32_t w = job.w, h = job.h, stride = job.stride;
-  Block b;
-  b.f = slot;
-  b.out = out;
-  b.w = w;
-  b.h = h;
-  b.pw = w + 2;
-  b.stride = stride;
-  b.pos = 0;
-  b.band = job.band_class;
-  b.style = job.style;
-  b.t = t;
-  b.tid = threadIdx.x;
-  for (uint32_t i = 0; i < (w + 2) * (h + 2); ++i) slot[i] = 0;
-  b.reset_contexts();
-  run_passes(b, job, segs, data);
-}
+// What a lane's next decision is.
+enum Step : uint32_t { kNext, kZero, kSign, kRefine, kRun, kUniform1, kUniform2, kSegSymbol };
 
 }  // namespace
 
@@ -513,45 +212,271 @@ struct QeTable {
   uint32_t e[47];
 };
 
-__global__ void __launch_bounds__(kClassicThreads) classic_kernel(const ClassicJob* __restrict__ jobs,
-                                                                  const ClassicSeg* __restrict__ segs, uint32_t njobs,
-                                                                  const uint8_t* __restrict__ arena,
-                                                                  const uint8_t* __restrict__ gather,
-                                                                  int32_t* __restrict__ coef, uint16_t* scratch,
-                                                                  uint32_t slot_words, uint32_t* queue, QeTable qt) {
+// The third-to-last group of parameters: slot_words, the 16-bit words of the
+// plan's largest block (classic_slot_words); lanes, the blocks each warp has
+// in flight (warps x lanes x slot_words at most kClassicPool).
+__global__ void __launch_bounds__(128) classic_kernel(const ClassicJob* __restrict__ jobs,
+                                                      const ClassicSeg* __restrict__ segs, uint32_t njobs,
+                                                      const uint8_t* __restrict__ arena,
+                                                      const uint8_t* __restrict__ gather, int32_t* __restrict__ coef,
+                                                      uint16_t* /*scratch*/, uint32_t slot_words, uint32_t* queue,
+                                                      QeTable qt, uint32_t lanes = 4) {
   __shared__ Tables t;
-  for (int i = threadIdx.x; i < 47; i += blockDim.x) t.qe[i] = qt.e[i];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    t.zc[0][i] = zc_context((uint8_t)i, kLlLh);
-    t.zc[1][i] = zc_context((uint8_t)i, kHl);
-    t.zc[2][i] = zc_context((uint8_t)i, kHh);
+  for (uint32_t i = threadIdx.x; i < 94; i += blockDim.x) {
+    const uint32_t e = qt.e[i >> 1], mps = i & 1;
+    const uint32_t nm = 2 * ((e >> 16) & 0x7Fu) + mps, nl = 2 * ((e >> 23) & 0x7Fu) + (mps ^ (e >> 30));
+    t.state[i] = (e & 0xFFFFu) | (nm << 16) | (nl << 23) | (mps << 31);
+  }
+  for (uint32_t i = threadIdx.x; i < 512; i += blockDim.x) {
+    const uint8_t n = window_byte(i);
+    t.zc[0][i] = zc_context(n, kLlLh);
+    t.zc[1][i] = zc_context(n, kHl);
+    t.zc[2][i] = zc_context(n, kHh);
+  }
+  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
     uint8_t label, xr;
-    sc_context((uint8_t)i, label, xr);
+    sc_context(sign_byte(i), label, xr);
     t.sc[i] = (uint8_t)(label | (xr << 7));
   }
   __syncthreads();
-  uint16_t* slot = scratch + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * slot_words;
+  const uint32_t lane = threadIdx.x & 31;
+  if (lane >= lanes) return;
+  const uint32_t id = (threadIdx.x >> 5) * lanes + lane;
+  uint16_t* const slot = t.cols + id * slot_words;
+
+  // The lane's block.
+  ClassicJob job;
+  job.passes = job.bitplanes = job.style = 0;
+  job.seg = 0;
+  uint32_t w = 0, h = 0, stride = 0, vcut = 0;
+  const uint8_t* data = nullptr;
+  uint32_t* out = nullptr;
+  const uint8_t* zc = t.zc[0];
+  // Its segments: passes [.., seg_end) come from the open decoder.
+  uint32_t nseg = 0, seg = 0, seg_end = 0, npasses = 0, off = 0;
+  bool raw = false;
+  MqDec dec;
+  dec.init_raw(nullptr, 0);
+  dec.c = dec.a = dec.ct = dec.b0 = dec.b1 = 0;
+  // Its position: pass, stripe, column, row, and the column words around it.
+  uint32_t pass = 0, kind = 0, one = 0, y0 = 0, x = 0, k = 0, rows = 0, cand = 0;
+  uint32_t L = 0, C = 0, R = 0, N = 0, old = 0, Q = 0;
+  int up = 0, down = 0;            // to the words above and below (0: none, or not to be seen)
+  uint32_t upm = 0, downm = 0;     // all ones where there are such words
+  uint32_t leave = 0;              // flags a column keeps when the pass leaves it
+  uint16_t* f = slot;              // the current column's word
+  uint32_t* col = nullptr;         // the current column's top sample
+  uint32_t step = kNext, label = 0, flip = 0, symbols = 0;
+  bool open = false;  // a block is being decoded
+  auto reset_contexts = [&]() {
+    for (int i = 0; i < 19; ++i) t.cx[i][id] = t.state[2 * initial_index(i)];
+  };
+  // The joined word of the column d after the current one (zero past the
+  // block's right edge).
+  auto column = [&](uint32_t d) -> uint32_t {
+    const bool in = x + d < w;
+    const uint16_t* p = f + (in ? d : 0);
+    const uint32_t v = join(p[up] & upm, p[0], p[down] & downm);
+    return in ? v : 0u;
+  };
+  auto stripe_begin = [&]() {
+    f = slot + (y0 >> 2) * w;
+    col = out + (size_t)y0 * stride;
+    rows = (1u << min(4u, h - y0)) - 1;
+    const bool above = y0 > 0, below = y0 + 4 < h && !vcut;
+    up = above ? -(int)w : 0;
+    upm = above ? ~0u : 0u;
+    down = below ? (int)w : 0;
+    downm = below ? ~0u : 0u;
+    x = 0;
+    L = 0;
+    old = C = column(0);
+    R = column(1);
+    N = column(2);
+  };
+  auto pass_begin = [&]() {
+    kind = pass % 3;
+    one = 1u << ((uint32_t)job.bitplanes - 1 - (pass + 2) / 3);
+    leave = kind == 0 ? ~kCodMask : ~0u;  // the cleanup pass ends the bit-plane
+    y0 = 0;
+    stripe_begin();
+  };
+  // The next pass, in its segment, or the next block's first pass; false
+  // when there is no block left.
+  auto next_pass = [&]() -> bool {
+    symbols = 0;
+    if (open) {
+      if (job.style & kReset) reset_contexts();
+      ++pass;
+    }
+    for (;;) {
+      if (open && pass < npasses && pass < seg_end) break;
+      if (open && seg < nseg && pass < npasses) {
+        // (Only with one segment per terminated run of passes.)
+        const ClassicSeg s = segs[job.seg + seg];
+        raw = !segment_is_arithmetic(job.style, seg_end);
+        if (raw) dec.init_raw(data + off, s.len);
+        else dec.init(data + off, s.len);
+        seg_end += s.passes;
+        off += s.len;
+        ++seg;
+        continue;
+      }
+      open = false;
+      const uint32_t j = atomicAdd(queue, 1u);
+      if (j >= njobs) return false;
+      job = jobs[j];
+      w = job.w;
+      h = job.h;
+      stride = job.stride;
+      out = reinterpret_cast<uint32_t*>(coef + job.dst);
+      if (((job.dst | stride | w) & 3) == 0) {
+        for (uint32_t y = 0; y < h; ++y)
+          for (uint32_t i = 0; i < w; i += 4)
+            *reinterpret_cast<uint4*>(out + (size_t)y * stride + i) = make_uint4(0, 0, 0, 0);
+      } else {
+        for (uint32_t y = 0; y < h; ++y)
+          for (uint32_t i = 0; i < w; ++i) out[(size_t)y * stride + i] = 0;
+      }
+      if (job.passes == 0 || job.bitplanes == 0) continue;
+      // The block's segments, in the input or (multi-layer) in the gather
+      // area.
+      data = (job.src & kClassicGathered) ? gather + (job.src & ~kClassicGathered) : arena + job.src;
+      const uint32_t words = w * ((h + 3) >> 2);
+      for (uint32_t i = 0; i < words; ++i) slot[i] = 0;
+      vcut = (job.style & kVCausal) ? 1 : 0;  // a stripe does not see the row below it
+      zc = t.zc[job.band_class];
+      reset_contexts();
+      npasses = 1 + 3 * ((uint32_t)job.bitplanes - 1);
+      pass = 0;
+      nseg = job.nseg;
+      seg = 0;
+      seg_end = 0;
+      off = 0;
+      raw = false;
+      if (!(job.style & (kBypass | kTermAll))) {
+        // One codeword for all passes.
+        uint32_t total = 0;
+        for (uint32_t i = 0; i < nseg; ++i) total += segs[job.seg + i].len;
+        dec.init(data, total);
+        npasses = min(npasses, (uint32_t)job.passes);
+        seg_end = npasses;
+        seg = nseg;
+      }
+      open = true;
+    }
+    pass_begin();
+    return true;
+  };
+
   for (;;) {
-    const uint32_t j = atomicAdd(queue, 1u);
-    if (j >= njobs) break;
-    decode_block(jobs[j], segs, arena, gather, coef, slot, &t);
+    // The next column of the stripe, when the current one is done.  (f stays
+    // inside the slot: the last column's step is undone by stripe_begin or
+    // next_pass, or reads nothing.)
+    const bool turn = step == kNext && cand == 0;
+    if (turn) {
+      C &= leave;
+      if (C != old) *f = own_word(C);
+      L = C;
+      old = C = R;
+      R = N;
+      ++x;
+      ++f;
+      ++col;
+      if (x >= w) {
+        // The next stripe, pass or block.
+        f = slot;
+        if (open && x == w && y0 + 4 < h) {
+          y0 += 4;
+          stripe_begin();
+        } else if (open && kind == 0 && (job.style & kSegSym) && symbols < 4) {
+          // Four uniform symbols end the cleanup pass.
+          step = kSegSymbol;
+          label = 18;
+          rows = 0;
+          old = C = 0;
+        } else if (!next_pass()) {
+          return;
+        }
+      } else {
+        N = column(2);
+      }
+    }
+    // The rows of this column that the pass codes.
+    const uint32_t own = C >> 1, around = L | C | R, any = around | (around >> 2) | ((L | R) >> 1);
+    const uint32_t all = (kind == 1 ? any : ~(C >> kCodBit)) & (kind == 2 ? own : ~own) & rows;
+    cand = turn ? all : cand;
+    Q = (L & 0x3Fu) | ((C & 0x3Fu) << 9) | ((R & 0x3Fu) << 18);
+    const bool run = turn && kind == 0 && all == 0xFu && Q == 0;
+    // The next sample of the column.
+    const bool pick = step == kNext && !run && cand != 0;
+    k = pick ? (uint32_t)__ffs((int)cand) - 1 : k;
+    cand &= pick ? cand - 1 : ~0u;
+    const uint32_t i = zc_index(Q, k);
+    const uint32_t refine = ((C >> (kRefBit + k)) & 1u) ? 16u : (i & ~kCentre) ? 15u : 14u;
+    const uint32_t zl = zc[i];
+    label = run ? 17u : pick ? (kind == 2 ? refine : zl) : label;
+    step = run ? (uint32_t)kRun : pick ? (kind == 2 ? (uint32_t)kRefine : (uint32_t)kZero) : step;
+    // Its decision (none when the column codes no sample).
+    uint32_t bit;
+    if (raw) {
+      bit = 0;
+      if (step != kNext) {
+        bit = raw_bit(dec.d, dec.len, dec.bp);
+        dec.bp = bit >> 1;
+        bit &= 1u;
+      }
+    } else {
+      uint32_t* const cx = &t.cx[label][id];
+      const uint32_t e = *cx;
+      bit = dec.decode(step == kNext ? 0u : e, cx, t.state);
+    }
+    const bool zero = step == kZero, sign = step == kSign, refined = step == kRefine;
+    const uint32_t s = bit ^ flip;  // (of a sign decision)
+    // A sample's value: its first magnitude bit with its sign, then the
+    // refinement bits added to it.
+    const bool neg = sign ? s != 0 : ((C >> (kSgnBit + 1 + k)) & 1u) != 0;
+    const uint32_t v = neg ? 0u - one : one;
+    uint32_t* const px = col + (size_t)(k * stride);
+    if (sign) *px = v;
+    if (refined && bit) atomicAdd(px, v);
+    const uint32_t set = sign ? 2u | (s << (kSgnBit + 1)) : refined ? 1u << kRefBit : zero && kind == 1 ? 1u << kCodBit : 0u;
+    C |= set << k;
+    // Significance propagation: the sample below has a neighbour now.
+    cand |= sign && kind == 1 ? (2u << k) & ~(C >> 1) & rows : 0u;
+    // The next step: a sign after a zero-coding 1 or the second uniform
+    // symbol (the rows after that one are then coded one by one), a run's
+    // uniform symbols, otherwise the next sample.
+    const bool u1 = step == kUniform1, u2 = step == kUniform2, ran = step == kRun;
+    k = u1 ? bit << 1 : u2 ? k | bit : k;
+    cand = ran ? 0u : u2 ? 0xFu & ~((2u << k) - 1) : cand;
+    symbols += step == kSegSymbol ? 1u : 0u;
+    const bool to_sign = (zero && bit) || u2;
+    const uint32_t next = ran && bit ? (uint32_t)kUniform1 : u1 ? (uint32_t)kUniform2 : (uint32_t)kNext;
+    step = to_sign ? (uint32_t)kSign : step == kSegSymbol && symbols < 4 ? (uint32_t)kSegSymbol : next;
+    const uint32_t e = t.sc[sign_index(L, C, R, k)];
+    flip = raw ? 0u : e >> 7;
+    label = to_sign ? e & 0x7Fu : 18u;
   }
 }
 
 cudaError_t launch_classic(const ClassicJob* jobs, const ClassicSeg* segs, uint32_t njobs, const uint8_t* arena,
-                           const uint8_t* gather, int32_t* coef, uint16_t* scratch, uint32_t slot_words, uint32_t ctas,
+                           const uint8_t* gather, int32_t* coef, uint32_t slot_words, uint32_t ctas, uint32_t lanes,
                            uint32_t* queue, cudaStream_t stream) {
   if (njobs == 0) return cudaSuccess;
-  if (!scratch || !queue || ctas == 0) return cudaErrorInvalidValue;
+  if (!queue || ctas == 0 || lanes == 0 || lanes > kClassicBlocks || lanes * slot_words > kClassicPool)
+    return cudaErrorInvalidValue;
   QeTable qt;
   for (int i = 0; i < 47; ++i)
     qt.e[i] = kQe[i] | ((uint32_t)kNmps[i] << 16) | ((uint32_t)kNlps[i] << 23) | ((uint32_t)kSwitch[i] << 30);
-  classic_kernel<<<ctas, kClassicThreads, 0, stream>>>(jobs, segs, njobs, arena, gather, coef, scratch, slot_words,
-                                                       queue, qt);
+  classic_kernel<<<ctas, kClassicThreads, 0, stream>>>(jobs, segs, njobs, arena, gather, coef, nullptr, slot_words,
+                                                       queue, qt, lanes);
   return cudaGetLastError();
 }
 
-uint32_t classic_threads_per_cta() { return kClassicThreads; }
+uint32_t classic_max_lanes(uint32_t slot_words) {
+  return std::max(1u, std::min(kClassicBlocks, kClassicPool / std::max(1u, slot_words)));
+}
 
 uint32_t classic_ctas_per_sm() {
   int n = 0;

@@ -1,0 +1,25 @@
+"""Classic (EBCOT) plans of enough code blocks that the lanes of a warp decode
+different blocks: every lane count up to 32, blocks of partial stripes and
+columns, each style's transitions, lossless against the source pixels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w,h,cb,cb_h,style", [
+    (64, 64, 0, 0, 0),      # 4 x 4 blocks: a few lanes of a few warps
+    (257, 131, 0, 0, 0),    # 6,500 blocks, ragged edges: eight lanes
+    (509, 303, 0, 0, 0x08),   # 29,000 blocks: 32 lanes, vertically causal
+    (509, 303, 0, 1, 0x05),   # 4 x 8, bypass and termination on every pass
+    (640, 253, 1, 0, 0x22),   # 8 x 4, context reset and segmentation symbols
+    (333, 1023, 4, 4, 0x2F),  # 64 x 64, every style at once
+])
+def test_many_blocks_lossless(w, h, cb, cb_h, style):
+    from signinum_b200 import encode
+    from signinum_b200.j2k_cuda import BackendRequest, Codec, PixelFormat
+
+    px = encode.he_rgb8(97 * w + h, w, h, 9.0)
+    cs = encode.encode_classic(px, w, h, 3, 8, style=style, levels=3, cb_exp=cb, cb_exp_h=cb_h)
+    s = Codec.decode_tile_to_device(cs, PixelFormat.Rgb8, BackendRequest.Cuda)
+    assert np.array_equal(np.frombuffer(s.to_bytes(), np.uint8), px)
