@@ -583,98 +583,124 @@ namespace {
 
 constexpr int kMsWarps = 8;  // warps (code blocks in flight) per CTA of the MagSgn pass
 
-// The lane's four stream bytes x (byte j at 8 j; zero past the segment) as
-// one bit string from the position of its first byte: byte j sits at
-// r_j = 8 j minus the 0xFF bytes among the lane's bytes before byte j - 1
-// and the byte before the lane (pf).  Bytes that follow an 0xFF carry 7 bits
-// (their top bit, a stuffed zero, overlaps the next byte and is ORed in as
-// the reference's reader does).  At most 32 bits: r_3 <= 24.
-__device__ __forceinline__ uint32_t lane_bits(uint32_t x, uint32_t pf, uint32_t f0, uint32_t f1) {
-  const uint32_t r1 = 8 - pf, r2 = r1 + 8 - f0, r3 = r2 + 8 - f1;
-  return (x & 0xFFu) | (((x >> 8) & 0xFFu) << r1) | (((x >> 16) & 0xFFu) << r2) | ((x >> 24) << r3);
-}
-
-// ORs a lane's bit string v into the bit array W at bit position pos (two
-// words at most).
-__device__ __forceinline__ void or_bits(uint32_t* W, uint32_t pos, uint32_t v) {
-  const uint32_t wi = pos >> 5, sh = pos & 31;
-  atomicOr(&W[wi], v << sh);
-  if (sh && (v >> (32 - sh))) atomicOr(&W[wi + 1], v >> (32 - sh));
+// 0x80 in every byte of x that is 0xFF (exact in each byte).
+__device__ __forceinline__ uint32_t ff_bytes(uint32_t x) {
+  const uint32_t y = ~x;
+  return ~(((y & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | y | 0x7F7F7F7Fu);
 }
 
 // Unstuffs the forward MagSgn byte stream [0, len) into a bit array W
 // (bit k of the stream = bit k%32 of W[k/32]): each byte contributes 8 bits,
 // or 7 after a 0xFF byte, ORed in at its offset exactly as the reference's
 // ForwardBitReader accumulates it (ht_block_decode.rs:888-930).  Bits past
-// the end read as ones (the reader pads with 0xFF).  Returns the number of
-// real bits.
+// the end, up to W[nwords - 1], read as ones (the reader pads with 0xFF).
 //
-// The warp takes 128 bytes per step, four per lane.  A step with no 0xFF
-// byte (and none just before it) is a plain bit shift of the input: each
-// lane stores one whole output word built from its word and its right
-// neighbour's.  Other steps place every byte at its own offset.
-__device__ uint32_t unstuff_magsgn(const uint8_t* src, uint32_t len, uint32_t* W, uint32_t nwords) {
-  const uint32_t lane = threadIdx.x & 31;
-  for (uint32_t i = lane; i < nwords; i += 32) W[i] = 0;
-  __syncwarp();
-  uint32_t ff_total = 0;  // 0xFF bytes among bytes [0, base)
-  uint32_t prev_ff = 0;   // byte base - 1 is 0xFF
-  for (uint32_t base = 0; base < len; base += 128) {
-    const uint32_t i0 = base + 4 * lane;
-    // Bytes i0 .. i0+3 (zero past len), little-endian.  Both aligned words
-    // hold a byte of the segment, so they lie inside its allocation.
-    uint32_t x = 0;
-    if (i0 < len) {
-      const uintptr_t addr = (uintptr_t)(src + i0);
-      const uint32_t* wp = reinterpret_cast<const uint32_t*>(addr & ~(uintptr_t)3);
-      const uint32_t sh = (uint32_t)(addr & 3);
-      const uint32_t nvalid = min(4u, len - i0);
-      const uint32_t lo = __ldg(wp);
-      const uint32_t hi = sh + nvalid > 4 ? __ldg(wp + 1) : 0u;
-      x = __funnelshift_r(lo, hi, 8 * sh);
-      if (nvalid < 4) x &= 0xFFFFFFFFu >> (8 * (4 - nvalid));
+// A group of G lanes (the warp, or each half-warp with its own stream; then
+// both run the longer one's steps) takes 8 G bytes per step, eight aligned
+// bytes per lane.  A lane removes the stuffed bits from its own bytes
+// (events, below), so that its bits are one string of n bits at bit P of the
+// stream, and writes the words of W whose first bit lies in its string, their
+// ends completed from the next lane's string by a shuffle: no word is written
+// twice but the first of a step, which lane 0 completes.  The pass is bound by
+// instruction issue: eight bytes per lane instead of four, one 64-bit load
+// instead of two unaligned words, plain stores instead of shared-memory
+// atomics into a zeroed array, and fewer operations per sample in the row
+// loops below took it from 2.70 to 2.17 ms on the uneven batch of 1,024 tiles
+// and from 0.50 to 0.41 ms on 256 tiles of 512 x 512.
+template <int G>
+__device__ __forceinline__ void unstuff_magsgn(const uint8_t* src, uint32_t len, uint32_t* W, uint32_t nwords) {
+  const uint32_t lane = threadIdx.x & 31, gl = lane & (G - 1), gsh = lane & (32 - G);
+  const uint32_t lt = (1u << gl) - 1;
+  const uint32_t lead = (uint32_t)((uintptr_t)src & 7);
+  const uint8_t* const base = src - lead;
+  const uint32_t span = lead + len;  // the stream is bytes [lead, span) from base
+  uint32_t steps = len ? (span + 8 * G - 1) / (8 * G) : 0;
+  if (G < 32) steps = max(steps, __shfl_xor_sync(0xFFFFFFFFu, steps, 16));
+  // The lane's eight bytes at offset o, zero outside the stream: one aligned
+  // load when all are in it, otherwise the aligned words that hold a byte of
+  // it (so they lie inside its allocation).
+  auto load = [&](uint32_t o) -> uint2 {
+    uint2 x = make_uint2(0, 0);
+    if (o >= lead && o + 8 <= span) {
+      x = __ldg(reinterpret_cast<const uint2*>(base + o));
+    } else if (o < span && len) {
+      const uint32_t first = o < lead ? lead - o : 0, last = min(span - o, 8u);
+      const uint32_t* wp = reinterpret_cast<const uint32_t*>(base + o);
+      if (first < 4) x.x = __ldg(wp);
+      if (last > 4) x.y = __ldg(wp + 1);
+      uint64_t v = ((uint64_t)x.y << 32) | x.x;
+      v = (v >> (8 * first)) << (8 * first);
+      if (last < 8) v &= (1ull << (8 * last)) - 1;
+      x = make_uint2((uint32_t)v, (uint32_t)(v >> 32));
     }
-    const uint32_t fm = i0 < len ? __vcmpeq4(x, 0xFFFFFFFFu) : 0u;  // 0xFF per 0xFF byte
-    // Padding bytes beyond len are zero, never 0xFF.
-    const bool full = base + 128 <= len;
-    if (full && !prev_ff && !__any_sync(0xFFFFFFFFu, fm != 0)) {
-      // Stream bit of byte base: 8 * base minus one per 0xFF before it.
-      const uint32_t P = 8 * base - ff_total;
-      const uint32_t s = P & 31, wb = P >> 5;
-      const uint32_t xn = __shfl_down_sync(0xFFFFFFFFu, x, 1);
-      if (lane < 31) W[wb + lane + 1] = __funnelshift_l(x, xn, s);
-      if (lane == 0) atomicOr(&W[wb], x << s);
-      if (lane == 31 && s) atomicOr(&W[wb + 32], x >> (32 - s));
-      continue;
+    return x;
+  };
+  uint32_t P = 0;     // stream bits before the step
+  uint32_t info = 0;  // of the byte before the step: bit 0 it is 0xFF, bit 1 its stuffed top bit is set
+  uint32_t end = 0;   // the lane's last string's end
+  uint2 x = load(8 * gl);
+  for (uint32_t k = 0; k < steps; ++k) {
+    const uint32_t o = 8 * (k * G + gl);
+    const uint2 nx = load(o + 8 * G);
+    const uint32_t first = o < lead ? lead - o : 0;
+    const uint32_t bytes = o < span ? min(span - o, 8u) - min(first, 8u) : 0u;
+    uint64_t v = ((uint64_t)x.y << 32) | x.x;
+    v >>= 8 * first;  // (first is not zero only on the lane that holds the stream's first byte)
+    uint32_t n = 8 * bytes, at = P + 8 * (o - min(o, 8 * G * k + (k ? 0u : lead)));
+    const uint32_t m0 = ff_bytes(x.x), m1 = ff_bytes(x.y);
+    if (__any_sync(0xFFFFFFFFu, (m0 | m1 | info) != 0)) {
+      // Positions: byte j of the stream is short when byte j - 1 is 0xFF, so
+      // a lane's string starts one bit earlier per 0xFF byte among those
+      // before the last byte before it.
+      const uint32_t count = (uint32_t)(__popc(m0) + __popc(m1));
+      uint32_t before = info & 1u;
+      for (uint32_t t = 1;; ++t) {
+        const uint32_t has = __ballot_sync(0xFFFFFFFFu, count >= t);
+        if (has == 0) break;
+        before += (uint32_t)__popc((has >> gsh) & lt);
+      }
+      const uint32_t mine = (m1 >> 31) | ((m1 >> 22) & (x.y >> 30) & 2u);
+      uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, mine, 1, G);
+      if (gl == 0) prev = info;
+      info = __shfl_sync(0xFFFFFFFFu, mine, G - 1, G);
+      at -= before - (prev & 1u);
+      // Events: a flag at each short byte of the lane's string.  Every bit
+      // above a short byte moves down by one; the byte's own top bit stays
+      // and is ORed with what arrives there.
+      uint64_t ev = (((uint64_t)m1 << 32) | m0) >> (8 * first);
+      ev = (ev << 8) | (prev & 1u ? 0x80u : 0u);
+      if (bytes < 8) ev &= (1ull << (8 * bytes)) - 1;
+      uint32_t drops = 0;
+      while (ev) {
+        const uint32_t top = (uint32_t)__ffsll((long long)ev) - drops;  // the short byte's end
+        ev &= ev - 1;
+        ++drops;
+        if (top < 64) v = (v & ((1ull << top) - 1)) | ((v >> top) << (top - 1));
+      }
+      n -= drops;
+      v |= (prev >> 1) & 1u;
     }
-    const uint32_t f0 = fm & 1, f1 = (fm >> 8) & 1, f2 = (fm >> 16) & 1, f3 = (fm >> 24) & 1;
-    const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, f0), b1 = __ballot_sync(0xFFFFFFFFu, f1);
-    const uint32_t b2 = __ballot_sync(0xFFFFFFFFu, f2), b3 = __ballot_sync(0xFFFFFFFFu, f3);
-    const uint32_t lt = (1u << lane) - 1;
-    // 0xFF bytes among [0, i0) and whether byte i0 - 1 is one.
-    const uint32_t F = ff_total + __popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt) + __popc(b3 & lt);
-    uint32_t pf = __shfl_up_sync(0xFFFFFFFFu, f3, 1);
-    if (lane == 0) pf = prev_ff;
-    // Byte i0 is shortened by the 0xFF bytes among [0, i0 - 1); the lane's
-    // other bytes follow it (lane_bits).
-    if (x) or_bits(W, 8 * i0 - (F - pf), lane_bits(x, pf, f0, f1));
-    ff_total += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
-    const uint32_t last = min(base + 128, len) - 1 - base;  // last byte of the step
-    const uint32_t lb = last >> 2, lj = last & 3;
-    const uint32_t lf = lj == 0 ? b0 : lj == 1 ? b1 : lj == 2 ? b2 : b3;
-    prev_ff = (lf >> lb) & 1;
+    uint32_t next = __shfl_down_sync(0xFFFFFFFFu, (uint32_t)v, 1, G);
+    if (gl == G - 1) next = 0;
+    __syncwarp();  // the previous step's words, before lane 0 completes the last of them
+    if (bytes) {
+      const uint32_t a = (0u - at) & 31u;  // bits of the string before its first own word
+      uint32_t* wp = W + ((at + 31) >> 5);
+      const uint64_t u = v >> a;
+      if (gl == 0 && a) wp[-1] |= (uint32_t)v << (32 - a);
+      if (a < n) wp[0] = (uint32_t)u | __funnelshift_lc(0u, next, n - a);
+      if (a + 32 < n) wp[1] = (uint32_t)(u >> 32) | __funnelshift_lc(0u, next, n - a - 32);
+      end = at + n;
+    }
+    P = __shfl_sync(0xFFFFFFFFu, at + n, G - 1, G);
+    x = nx;
   }
-  // Real bits: 8 per byte minus one per byte that follows a 0xFF.
-  const uint32_t end_bits = len ? 8 * len - (ff_total - prev_ff) : 0;
+  const uint32_t bits = __shfl_sync(0xFFFFFFFFu, end, len ? ((span - 1) >> 3) & (G - 1) : 0, G);
   __syncwarp();
-  // Padding: every bit from end_bits on is one.
-  for (uint32_t wi = lane; wi < nwords; wi += 32) {
-    uint32_t lo = wi * 32;
-    if (lo >= end_bits) W[wi] = 0xFFFFFFFFu;
-    else if (lo + 32 > end_bits) W[wi] |= 0xFFFFFFFFu << (end_bits - lo);
-  }
+  // Padding: every bit from there on is one.
+  if (gl == 0 && (bits & 31) && (bits >> 5) < nwords) W[bits >> 5] |= 0xFFFFFFFFu << (bits & 31);
+  for (uint32_t wi = ((bits + 31) >> 5) + gl; wi < nwords; wi += G) W[wi] = 0xFFFFFFFFu;
   __syncwarp();
-  return end_bits;
 }
 
 __device__ __forceinline__ uint32_t bits_at(const uint32_t* W, uint32_t nwords, uint32_t off) {
@@ -696,8 +722,7 @@ __device__ __forceinline__ uint32_t spread4(uint32_t x) { return (x * 0x00204081
 
 struct QuadBits {
   uint32_t m;    // m_n per sample: U - e_k when significant, else 0
-  uint32_t cs;   // per sample, the bits of the samples before it in the quad
-  uint32_t tot;  // the quad's bits
+  uint32_t incl; // per sample, the bits up to its own end in the quad
 };
 
 // U is the quad's u_q (plus the exponent bound kappa after the first row);
@@ -707,31 +732,49 @@ struct QuadBits {
 __device__ __forceinline__ QuadBits quad_bits(uint32_t inf, uint32_t U) {
   const uint32_t sig = spread4((inf >> 4) & 0xFu), k = spread4(inf >> 12);
   const uint32_t m = (min(U, 31u) * 0x01010101u - k) & (sig * 0xFFu);
-  const uint32_t incl = m * 0x01010101u;
-  return QuadBits{m, incl - m, incl >> 24};
+  return QuadBits{m, m * 0x01010101u};
 }
 
-// The 32 stream bits from bit c (< 64) of the 64-bit window hi:lo.
-__device__ __forceinline__ uint32_t window_bits(uint32_t lo, uint32_t hi, uint32_t c) {
-  return (uint32_t)((((uint64_t)hi << 32) | lo) >> c);
+// Inclusive prefix sum over the calling group of G lanes (the warp or a
+// half-warp): the shuffle's own in-range predicate guards each addition.
+template <int G>
+__device__ __forceinline__ uint32_t inclusive_scan(uint32_t x) {
+#ifdef __CUDA_ARCH__
+#pragma unroll
+  for (int d = 1; d < G; d <<= 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .u32 t;\n\t"
+        "shfl.sync.up.b32 t|p, %0, %1, %2, 0xffffffff;\n\t"
+        "@p add.u32 %0, %0, t;\n\t}"
+        : "+r"(x)
+        : "r"(d), "r"((32 - G) << 8));
+#else
+  const uint32_t gl = threadIdx.x & (G - 1);
+  for (int d = 1; d < G; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, x, d, G);
+    if (gl >= (uint32_t)d) x += v;
+  }
+#endif
+  return x;
 }
 
 // Sample i's coefficient from its bits msv (sign first, then the magnitude
-// bits below the implied ones), bit count m, known-1 bit e1 and
-// significance: decode_mag_sgn_sample_with_vn's v_n (ht_block_decode.rs:1010-1032)
+// bits below the implied ones), bit count m (low five bits), known-1 bit e1
+// and significance: decode_mag_sgn_sample_with_vn's v_n (ht_block_decode.rs:1010-1032)
 // gives the sign-magnitude word sign << 31 | (v + 2) << (p - 1) in 32-bit
 // arithmetic (whose top bit, in the largest valid magnitudes, the shift can
 // set as well); RAW returns that word, otherwise coefficient_to_i32
 // (:225-234) of it: (word & 0x7FFFFFFF) >> (31 - nbp), negated when the top
 // bit is set, computed as (word << 1) >> rs with rs = 32 - nbp (1 when
-// nbp >= 31; the shift clamps at 32).  E receives the bit length of v (0
-// when insignificant), the exponent the row below needs.
+// nbp >= 31; the shift clamps at 32).  E receives the position of v's top bit
+// (one less than its bit length; 0 when insignificant), the exponent the row
+// below needs.
 template <bool RAW>
 __device__ __forceinline__ int32_t sample_value(uint32_t msv, uint32_t m, uint32_t e1, bool sig, uint32_t p,
                                                 uint32_t rs, uint32_t& E) {
-  const uint32_t mask = __funnelshift_lc(0xFFFFFFFFu, 0u, m);
-  const uint32_t v = (msv & mask) | (e1 << m) | 1u;
-  E = sig ? 32 - __clz(v) : 0u;
+  const uint32_t mask = __funnelshift_l(0xFFFFFFFFu, 0u, m);
+  const uint32_t v = (msv & mask) | __funnelshift_l(0u, e1, m) | 1u;
+  E = sig ? 31u - (uint32_t)__clz(v) : 0u;
   const uint32_t word = (msv << 31) | ((v + 2) << (p - 1));
   if (RAW) return sig ? (int32_t)word : 0;
   const int32_t mag = (int32_t)__funnelshift_rc(word << 1, 0u, rs);
@@ -740,29 +783,34 @@ __device__ __forceinline__ int32_t sample_value(uint32_t msv, uint32_t m, uint32
 
 // The four samples of a quad whose stream bits start at `off`: one clamped
 // three-word window read serves all four when the quad holds fewer than 64
-// bits; otherwise each sample reads its own 32 bits.
+// bits, each sample's bits shifted out after it; otherwise each sample reads
+// its own 32 bits.
 template <bool RAW>
 __device__ __forceinline__ void quad_samples(const uint32_t* W, uint32_t ms_words, uint32_t lim, uint32_t off,
                                              uint32_t inf, const QuadBits& qb, uint32_t p, uint32_t rs,
                                              int32_t val[4], uint32_t E[4]) {
   uint32_t lo, hi;
   {
-    const uint32_t o = min(off, lim), wi = o >> 5, sh = o & 31;
+    const uint32_t o = min(off, lim), wi = o >> 5;
     const uint32_t a0 = W[wi], a1 = W[wi + 1], a2 = W[wi + 2];
-    lo = __funnelshift_r(a0, a1, sh);
-    hi = __funnelshift_r(a1, a2, sh);
+    lo = __funnelshift_r(a0, a1, o);
+    hi = __funnelshift_r(a1, a2, o);
   }
   uint32_t msv[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) msv[i] = window_bits(lo, hi, (qb.cs >> (8 * i)) & 0xFFu);
-  if (qb.tot >= 64) {
+  for (int i = 0; i < 4; ++i) {
+    msv[i] = lo;
+    // (Shift counts are taken modulo 32: the sample's byte of m.)
+    lo = __funnelshift_r(lo, hi, qb.m >> (8 * i));
+    hi = __funnelshift_r(hi, 0u, qb.m >> (8 * i));
+  }
+  if ((qb.incl >> 24) >= 64) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) msv[i] = bits_at(W, ms_words, off + ((qb.cs >> (8 * i)) & 0xFFu));
+    for (int i = 0; i < 4; ++i) msv[i] = bits_at(W, ms_words, off + (((qb.incl - qb.m) >> (8 * i)) & 0xFFu));
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    val[i] = sample_value<RAW>(msv[i], (qb.m >> (8 * i)) & 0xFFu, (inf >> (8 + i)) & 1u, (inf >> (4 + i)) & 1u, p,
-                               rs, E[i]);
+    val[i] = sample_value<RAW>(msv[i], qb.m >> (8 * i), (inf >> (8 + i)) & 1u, (inf >> (4 + i)) & 1u, p, rs, E[i]);
 }
 
 
@@ -798,13 +846,13 @@ __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_wor
   const uint32_t lim = 32 * (ms_words - 3);
   const bool pairs = ((job.dst | stride) & 1) == 0;  // 8-byte aligned sample pairs
   const uint32_t nq = (w + 1) / 2, qs = sym_row_stride(w);
-  uint8_t* Eprev = Ebase;  // wide blocks: bit lengths of v_n per column + 1, row above
+  uint8_t* Eprev = Ebase;  // wide blocks: top bit positions of v_n per column + 1, row above
   uint8_t* Ecur = Ebase + cols;
   if (!NARROW) {
     for (uint32_t c = lane; c < cols; c += 32) Eprev[c] = 0;
     __syncwarp();
   }
-  uint32_t e_left = 0, e_right = 0;  // NARROW: bottom-row bit lengths of this lane's quad
+  uint32_t e_left = 0, e_right = 0;  // NARROW: bottom-row top bit positions of this lane's quad
   uint32_t rowbase = 0;
   bool bad = false;
   // Running pointers: sample row y of the block and quad row r of its symbols.
@@ -830,12 +878,11 @@ __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_wor
       if (!initial) {
         uint32_t e;
         if (NARROW) {
-          // Columns 2q-1 and 2q+2 belong to the neighbouring lanes' quads;
-          // outside the block they are zero (lanes past nq hold zeros).
-          uint32_t l = __shfl_up_sync(0xFFFFFFFFu, e_right, 1);
-          uint32_t rr = __shfl_down_sync(0xFFFFFFFFu, e_left, 1);
-          if (lane == 0) l = 0;
-          if (lane == 31) rr = 0;
+          // Columns 2q-1 and 2q+2 belong to the neighbouring lanes' quads
+          // (lanes past nq hold zeros; the first and last lane's shuffles
+          // give them their own samples, which the maximum has anyway).
+          const uint32_t l = __shfl_up_sync(0xFFFFFFFFu, e_right, 1);
+          const uint32_t rr = __shfl_down_sync(0xFFFFFFFFu, e_left, 1);
           e = max(max(l, e_left), max(e_right, rr));
         } else {
           // Columns 2q-1 .. 2q+2 of the row above live at Eprev[col + 1]
@@ -844,22 +891,19 @@ __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_wor
                            max((uint32_t)Eprev[2 * q + 2], (uint32_t)Eprev[2 * q + 3]))
                      : 0;
         }
+        // kappa: max(bit length, 2) - 1 of the samples above when at least
+        // two of the quad's are significant, else 1.
         uint32_t gamma = inf & 0xF0;
         gamma &= gamma - 0x10;
-        if (active) U += gamma != 0 ? max(e, 2u) - 1 : 1;
+        U += gamma != 0 ? max(e, 1u) : 1u;
       }
-      bad |= active && U > mmsbp2;
+      // (A lane without a quad holds U of 0 or 1 and no significant sample.)
+      bad |= U > mmsbp2;
       const QuadBits qb = quad_bits(inf, U);
-      // Warp inclusive scan of the bit counts.
-      uint32_t inc = qb.tot;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, d);
-        if (lane >= (uint32_t)d) inc += v;
-      }
-      const uint32_t chunk_bits = __shfl_sync(0xFFFFFFFFu, inc, 31);
-      const uint32_t off = rowbase + inc - qb.tot;
-      rowbase += chunk_bits;
+      const uint32_t tot = qb.incl >> 24;
+      const uint32_t inc = inclusive_scan<32>(tot);
+      const uint32_t off = rowbase + inc - tot;
+      rowbase += __shfl_sync(0xFFFFFFFFu, inc, 31);
       int32_t val[4];
       uint32_t E[4];
       quad_samples<RAW>(W, ms_words, lim, off, inf, qb, p, rs, val, E);
@@ -908,88 +952,11 @@ __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_wor
 
 // Narrow blocks (at most 32 wide: 16 quads a row) would leave half of a
 // warp idle, so a warp takes two of them, one per half-warp (lanes 0-15 and
-// 16-31).  The functions below are unstuff_magsgn and magsgn_rows for that
-// case: every shuffle, ballot and scan runs on all 32 lanes with the
+// 16-31).  The function below is magsgn_rows for that case (and unstuff_magsgn
+// has its half-warp form): every shuffle, ballot and scan runs on all 32 lanes with the
 // half-warp as its segment, and both halves run the longer block's loop
 // trip counts (a half past its own work idles), so no warp-synchronous
 // operation sits in a branch that one half skips.
-
-// unstuff_magsgn for the calling half-warp's stream: 64 bytes per step.
-__device__ uint32_t unstuff_half(const uint8_t* src, uint32_t len, uint32_t* W, uint32_t nwords) {
-  const uint32_t lane = threadIdx.x & 31, gl = lane & 15, gsh = lane & 16;
-  for (uint32_t i = gl; i < nwords; i += 16) W[i] = 0;
-  __syncwarp();
-  const uint32_t steps = (len + 63) / 64;
-  const uint32_t nsteps = max(steps, __shfl_xor_sync(0xFFFFFFFFu, steps, 16));
-  uint32_t ff_total = 0;  // 0xFF bytes among bytes [0, base)
-  uint32_t prev_ff = 0;   // byte base - 1 is 0xFF
-  for (uint32_t k = 0; k < nsteps; ++k) {
-    const uint32_t base = 64 * k, i0 = base + 4 * gl;
-    uint32_t x = 0;
-    if (i0 < len) {
-      const uintptr_t addr = (uintptr_t)(src + i0);
-      const uint32_t* wp = reinterpret_cast<const uint32_t*>(addr & ~(uintptr_t)3);
-      const uint32_t sh = (uint32_t)(addr & 3);
-      const uint32_t nvalid = min(4u, len - i0);
-      const uint32_t lo = __ldg(wp);
-      const uint32_t hi = sh + nvalid > 4 ? __ldg(wp + 1) : 0u;
-      x = __funnelshift_r(lo, hi, 8 * sh);
-      if (nvalid < 4) x &= 0xFFFFFFFFu >> (8 * (4 - nvalid));
-    }
-    const uint32_t fm = i0 < len ? __vcmpeq4(x, 0xFFFFFFFFu) : 0u;
-    // One vote first: a step in which neither half has an 0xFF byte (and no
-    // 0xFF byte just before it) is a plain shift of the input in both, and
-    // needs neither the per-byte votes nor the 0xFF counts.
-    const uint32_t any_ff = (__ballot_sync(0xFFFFFFFFu, fm != 0) >> gsh) & 0xFFFFu;  // every lane votes
-    const bool plain = base >= len || (base + 64 <= len && !prev_ff && any_ff == 0);
-    if (__all_sync(0xFFFFFFFFu, plain)) {
-      const uint32_t xn = __shfl_down_sync(0xFFFFFFFFu, x, 1, 16);
-      if (base < len) {
-        const uint32_t P = 8 * base - ff_total;
-        const uint32_t s = P & 31, wb = P >> 5;
-        if (gl < 15) W[wb + gl + 1] = __funnelshift_l(x, xn, s);
-        if (gl == 0) atomicOr(&W[wb], x << s);
-        if (gl == 15 && s) atomicOr(&W[wb + 16], x >> (32 - s));
-      }
-      continue;
-    }
-    const uint32_t f0 = fm & 1, f1 = (fm >> 8) & 1, f2 = (fm >> 16) & 1, f3 = (fm >> 24) & 1;
-    const uint32_t b0 = (__ballot_sync(0xFFFFFFFFu, f0) >> gsh) & 0xFFFFu;
-    const uint32_t b1 = (__ballot_sync(0xFFFFFFFFu, f1) >> gsh) & 0xFFFFu;
-    const uint32_t b2 = (__ballot_sync(0xFFFFFFFFu, f2) >> gsh) & 0xFFFFu;
-    const uint32_t b3 = (__ballot_sync(0xFFFFFFFFu, f3) >> gsh) & 0xFFFFu;
-    const uint32_t xn = __shfl_down_sync(0xFFFFFFFFu, x, 1, 16);
-    uint32_t pf = __shfl_up_sync(0xFFFFFFFFu, f3, 1, 16);
-    if (base < len) {
-      if (base + 64 <= len && !prev_ff && (b0 | b1 | b2 | b3) == 0) {
-        const uint32_t P = 8 * base - ff_total;
-        const uint32_t s = P & 31, wb = P >> 5;
-        if (gl < 15) W[wb + gl + 1] = __funnelshift_l(x, xn, s);
-        if (gl == 0) atomicOr(&W[wb], x << s);
-        if (gl == 15 && s) atomicOr(&W[wb + 16], x >> (32 - s));
-      } else {
-        const uint32_t lt = (1u << gl) - 1;
-        const uint32_t F = ff_total + __popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt) + __popc(b3 & lt);
-        if (gl == 0) pf = prev_ff;
-        if (x) or_bits(W, 8 * i0 - (F - pf), lane_bits(x, pf, f0, f1));
-      }
-      ff_total += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
-      const uint32_t last = min(base + 64, len) - 1 - base;  // last byte of the step
-      const uint32_t lb = last >> 2, lj = last & 3;
-      const uint32_t lf = lj == 0 ? b0 : lj == 1 ? b1 : lj == 2 ? b2 : b3;
-      prev_ff = (lf >> lb) & 1;
-    }
-  }
-  const uint32_t end_bits = len ? 8 * len - (ff_total - prev_ff) : 0;
-  __syncwarp();
-  for (uint32_t wi = gl; wi < nwords; wi += 16) {
-    uint32_t lo = wi * 32;
-    if (lo >= end_bits) W[wi] = 0xFFFFFFFFu;
-    else if (lo + 32 > end_bits) W[wi] |= 0xFFFFFFFFu << (end_bits - lo);
-  }
-  __syncwarp();
-  return end_bits;
-}
 
 // magsgn_rows<true, false> for the calling half-warp's block (live) over
 // hmax rows, the taller of the two blocks' heights.  Returns true on the
@@ -1020,26 +987,19 @@ __device__ bool magsgn_rows_half(const HtJob& job, bool live, const uint32_t* W,
     const uint32_t inf = s & 0xFFFF;
     uint32_t U = s >> 16;
     if (!initial) {
-      uint32_t l = __shfl_up_sync(0xFFFFFFFFu, e_right, 1, 16);
-      uint32_t rr = __shfl_down_sync(0xFFFFFFFFu, e_left, 1, 16);
-      if (gl == 0) l = 0;
-      if (gl == 15) rr = 0;
+      const uint32_t l = __shfl_up_sync(0xFFFFFFFFu, e_right, 1, 16);
+      const uint32_t rr = __shfl_down_sync(0xFFFFFFFFu, e_left, 1, 16);
       const uint32_t e = max(max(l, e_left), max(e_right, rr));
       uint32_t gamma = inf & 0xF0;
       gamma &= gamma - 0x10;
-      if (active) U += gamma != 0 ? max(e, 2u) - 1 : 1;
+      U += gamma != 0 ? max(e, 1u) : 1u;
     }
-    bad |= active && U > mmsbp2;
+    bad |= U > mmsbp2;
     const QuadBits qb = quad_bits(inf, U);
-    uint32_t inc = qb.tot;
-#pragma unroll
-    for (int d = 1; d < 16; d <<= 1) {
-      uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, d, 16);
-      if (gl >= (uint32_t)d) inc += v;
-    }
-    const uint32_t chunk_bits = __shfl_sync(0xFFFFFFFFu, inc, 15, 16);
-    const uint32_t off = rowbase + inc - qb.tot;
-    rowbase += chunk_bits;
+    const uint32_t tot = qb.incl >> 24;
+    const uint32_t inc = inclusive_scan<16>(tot);
+    const uint32_t off = rowbase + inc - tot;
+    rowbase += __shfl_sync(0xFFFFFFFFu, inc, 15, 16);
     int32_t val[4];
     uint32_t E[4];
     quad_samples<false>(W, ms_words, lim, off, inf, qb, p, rs, val, E);
@@ -1115,7 +1075,7 @@ __device__ void magsgn_block(const HtJob& job, const uint8_t* __restrict__ arena
     // and reads beyond them return ones, so bits past the end still read as
     // the reference's 0xFF padding.
     const uint32_t words = (ms_len + 15) / 4 + 2;
-    unstuff_magsgn(src, ms_len, W, words);
+    unstuff_magsgn<32>(src, ms_len, W, words);
     // Blocks with refinement passes keep the sign-magnitude words for them.
     const bool raw = job.passes > 1;
     const bool bad =
@@ -1165,7 +1125,7 @@ __device__ void magsgn_pair(const HtJob* __restrict__ jobs, uint32_t a, uint32_t
       words = (ms_len + 15) / 4 + 2;
     }
   }
-  unstuff_half(src, ms_len, Wg, words);
+  unstuff_magsgn<16>(src, ms_len, Wg, words);
   const uint32_t hh = ok ? job.h : 0;
   const uint32_t hmax = max(hh, __shfl_xor_sync(0xFFFFFFFFu, hh, 16));
   const bool bad = magsgn_rows_half(job, ok, Wg, words, hmax, sym, dst);
