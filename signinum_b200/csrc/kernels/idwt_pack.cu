@@ -18,15 +18,16 @@
 // they need).  The vertical pass streams down the rows keeping the previous
 // odd row and the previous updated even row in registers.  Symmetric
 // extension is done by reflecting row/column indices (it commutes with the
-// lifting steps), so the edges need no special arithmetic.  No barriers.
+// lifting steps): the lanes' column offsets are reflected once per unit, so
+// the edges run the same code.  No barriers.
 //
 // The last level keeps the streams of all components of a pixel in the same
 // lane and finishes the pixels there: inverse RCT (mct.rs:117-150),
 // +2^(bd-1) (decode.rs:1720-1729, :1748-1752) and the conversion to the
 // requested pixel format (crates/signinum-j2k-native/src/lib.rs:1772-1840,
 // :2202-2294; crates/signinum-j2k/src/decode.rs:345-356, :517-545); each lane
-// packs its four pixels into 32-bit words, the words of a row are staged per
-// warp in shared memory and the row is written with 16-byte stores.
+// packs its four pixels into 32-bit words and stores them itself, or through
+// the warp's row buffer where the row does not fall on lane boundaries.
 #include <algorithm>
 #include <cstdint>
 
@@ -39,13 +40,17 @@ namespace {
 constexpr int kLanes = 32;
 static_assert(kIdwtStripW == 4 * kLanes, "one strip is four columns per lane");
 
-// Periodic symmetric extension of index i into [0, n) (reflections about the
-// first and last samples; the streams overshoot by at most a few samples).
-__device__ __forceinline__ int fold(int i, int n) {
+// Whole-sample symmetric extension of index i into [0, n).  Reflection keeps
+// an index's parity; indices far outside (columns of lanes past a narrow
+// level) end at the nearest in-range index of the same parity, so the band
+// they select (low for even, high for odd) and the place in it stay in bounds.
+__device__ __forceinline__ int reflect(int i, int n) {
   if ((unsigned)i < (unsigned)n) return i;
   if (n == 1) return 0;
 #pragma unroll 1
-  for (int k = 0; k < 8 && (i < 0 || i >= n); ++k) i = i < 0 ? -i : 2 * (n - 1) - i;
+  for (int k = 0; k < 4 && (unsigned)i >= (unsigned)n; ++k) i = i < 0 ? -i : 2 * (n - 1) - i;
+  if (i < 0) return i & 1;
+  if (i >= n) return (n - 1) - (((n - 1) ^ i) & 1);
   return i;
 }
 
@@ -54,115 +59,119 @@ struct Bands {
   const int32_t* hl;
   const int32_t* lh;
   const int32_t* hh;
+};
+
+// Whether every band row of a level of width w starts 8-byte aligned.
+__device__ __forceinline__ bool aligned_bands(const Bands& B, int w) {
+  const uintptr_t a = (uintptr_t)B.ll | (uintptr_t)B.hl | (uintptr_t)B.lh | (uintptr_t)B.hh;
+  return (w & 3) == 0 && (a & 7) == 0;
+}
+
+// A lane's columns of a level: band offsets of its image columns c .. c+3
+// (low band l0, l1; high band h0, h1), and of the samples the strip's edge
+// lanes need besides: lane 0 the high band left of its columns (xh), lane 31
+// the low and high band right of them (xl, xh).  Whole strips of a level
+// whose rows are 8-byte aligned (VEC) read the pairs with one load each; at
+// the level's edges their extra samples are among the lane's own.
+struct Cols {
   int w, h;
-  bool vec;  // w % 4 == 0 and 8-byte aligned bases: every band row starts 8-byte aligned
+  int l0, l1, h0, h1, xl, xh;
+  bool left, right;  // VEC: lane 0 (31) has a sample to load on its left (right)
 };
 
-__device__ __forceinline__ Bands make_bands(const int32_t* ll, const int32_t* hl, const int32_t* lh,
-                                            const int32_t* hh, int w, int h) {
-  const uintptr_t a = (uintptr_t)ll | (uintptr_t)hl | (uintptr_t)lh | (uintptr_t)hh;
-  return Bands{ll, hl, lh, hh, w, h, (w & 3) == 0 && (a & 7) == 0};
+// *p where `go` holds, else 0: a predicated load, so that the loads around it
+// stay in one batch.
+__device__ __forceinline__ int load_if(bool go, const int32_t* p) {
+#ifdef __CUDA_ARCH__
+  int v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.b32 %0, [%1];\n\t}"
+      : "=r"(v)
+      : "l"(p), "r"((uint32_t)go));
+  return v;
+#else
+  return go ? *p : 0;
+#endif
 }
 
-// Band samples of one interleaved row at this lane's band columns b, b + 1
-// (image columns 2b .. 2b+3), plus the extra samples the strip's edge lanes
-// need.  Loads only: lifting happens in lift_row, so a caller can keep the
-// next rows' loads in flight while it lifts the current ones.
-struct RawRow {
-  int lo0, lo1, hi0, hi1;  // low / high band at columns b, b + 1
-  int x1;                  // lane 0: high band at column b - 1; lane 31: low band at column b + 2
-  int x2;                  // lane 31: high band at column b + 2
-};
-
-// INTERIOR: the strip starts at column 128 or later and ends at least two
-// columns before the level's right edge (interior_strip), so every lane's
-// columns and the edge lanes' extra samples lie inside the level and no
-// column needs a bounds test or a mirror.
-__device__ __forceinline__ bool interior_strip(int x0, int w) {
-  return x0 >= (int)kIdwtStripW && x0 + (int)kIdwtStripW + 2 <= w;
-}
-
-template <bool INTERIOR = false>
-__device__ __forceinline__ RawRow load_row(const Bands& B, int y, int b, int lane) {
-  y = fold(y, B.h);
-  const int r = y >> 1;
-  const int lw = (B.w + 1) >> 1, hw = B.w >> 1;
-  const int32_t* Lr = ((y & 1) ? B.lh : B.ll) + (size_t)r * lw;
-  const int32_t* Hr = ((y & 1) ? B.hh : B.hl) + (size_t)r * hw;
-  RawRow R;
-  if (INTERIOR) {
-    if (B.vec) {
-      const int2 l = __ldg(reinterpret_cast<const int2*>(Lr + b));
-      const int2 h = __ldg(reinterpret_cast<const int2*>(Hr + b));
-      R.lo0 = l.x;
-      R.lo1 = l.y;
-      R.hi0 = h.x;
-      R.hi1 = h.y;
-    } else {
-      R.lo0 = __ldg(Lr + b);
-      R.lo1 = __ldg(Lr + b + 1);
-      R.hi0 = __ldg(Hr + b);
-      R.hi1 = __ldg(Hr + b + 1);
-    }
-    R.x1 = lane == 0 ? __ldg(Hr + b - 1) : lane == kLanes - 1 ? __ldg(Lr + b + 2) : 0;
-    R.x2 = lane == kLanes - 1 ? __ldg(Hr + b + 2) : 0;
-    return R;
+template <bool VEC>
+__device__ __forceinline__ Cols make_cols(int x0, int w, int h, int lane) {
+  Cols o;
+  const int c = x0 + 4 * lane;
+  o.w = w;
+  o.h = h;
+  if (VEC) {
+    o.l0 = o.h0 = c >> 1;
+    o.l1 = o.h1 = 0;
+    o.left = lane == 0 && x0 > 0;
+    o.right = lane == kLanes - 1 && x0 + kIdwtStripW < w;
+    o.xl = 2;
+    o.xh = o.left ? -1 : 2;  // from the pair
+  } else {
+    o.l0 = reflect(c, w) >> 1;
+    o.h0 = reflect(c + 1, w) >> 1;
+    o.l1 = reflect(c + 2, w) >> 1;
+    o.h1 = reflect(c + 3, w) >> 1;
+    o.xl = reflect(c + 4, w) >> 1;
+    o.xh = reflect(lane == 0 ? c - 1 : c + 5, w) >> 1;
+    o.left = o.right = false;
   }
-  if (B.vec && b + 1 < hw) {
-    // b is even and both band widths are even: one 8-byte load per band.
-    const int2 l = __ldg(reinterpret_cast<const int2*>(Lr + b));
-    const int2 h = __ldg(reinterpret_cast<const int2*>(Hr + b));
+  return o;
+}
+
+// Band samples of one interleaved row at this lane's columns.  Loads only:
+// lifting happens in lift_row, so a caller can keep the next rows' loads in
+// flight while it lifts the current ones.
+struct RawRow {
+  int lo0, lo1, hi0, hi1;  // low / high band at columns c, c+2 / c+1, c+3
+  int xl, xh;              // edge lanes: Cols::xl, Cols::xh
+};
+
+// Row r of the low and the high band.
+template <bool VEC>
+__device__ __forceinline__ RawRow load_row(const int32_t* low, const int32_t* high, int r, const Cols& o, int lane) {
+  const int32_t* Lr = low + (size_t)r * ((o.w + 1) >> 1);
+  const int32_t* Hr = high + (size_t)r * (o.w >> 1);
+  RawRow R;
+  if (VEC) {
+    Lr += o.l0;
+    Hr += o.h0;
+    const int2 l = __ldg(reinterpret_cast<const int2*>(Lr));
+    const int2 h = __ldg(reinterpret_cast<const int2*>(Hr));
     R.lo0 = l.x;
     R.lo1 = l.y;
     R.hi0 = h.x;
     R.hi1 = h.y;
-  } else {
-    R.lo0 = b < lw ? __ldg(Lr + b) : 0;
-    R.lo1 = b + 1 < lw ? __ldg(Lr + b + 1) : 0;
-    R.hi0 = b < hw ? __ldg(Hr + b) : 0;
-    R.hi1 = b + 1 < hw ? __ldg(Hr + b + 1) : 0;
+    R.xh = load_if(o.left || o.right, Hr + o.xh);
+    R.xl = load_if(o.right, Lr + 2);
+    return R;
   }
-  R.x1 = (lane == 0 && b > 0) ? __ldg(Hr + b - 1) : (lane == kLanes - 1 && b + 2 < lw) ? __ldg(Lr + b + 2) : 0;
-  R.x2 = (lane == kLanes - 1 && b + 2 < hw) ? __ldg(Hr + b + 2) : 0;
+  R.lo0 = __ldg(Lr + o.l0);
+  R.lo1 = __ldg(Lr + o.l1);
+  R.hi0 = R.hi1 = R.xl = R.xh = 0;
+  if (o.w > 1) {
+    R.hi0 = __ldg(Hr + o.h0);
+    R.hi1 = __ldg(Hr + o.h1);
+    if (lane == 0 || lane == kLanes - 1) {
+      R.xh = __ldg(Hr + o.xh);
+      R.xl = __ldg(Lr + o.xl);
+    }
+  }
   return R;
 }
 
-// Horizontal lifting of a loaded row: samples of image columns 2b .. 2b+3
-// (x: 2b, y: 2b+1, z: 2b+2, w: 2b+3).  Columns past the right edge return
-// garbage.  X[-1] mirrors X[1] and X[w] mirrors X[w-2].
-template <bool INTERIOR = false>
-__device__ __forceinline__ int4 lift_row(const RawRow& R, int w, int b, int lane) {
-  if (INTERIOR) {
-    int hm1 = __shfl_up_sync(0xFFFFFFFFu, R.hi1, 1);  // X[c-1]
-    if (lane == 0) hm1 = R.x1;
-    const int h0 = R.hi0, h1 = R.hi1;                  // X[c+1], X[c+3]
-    const int e0 = R.lo0 - ((hm1 + h0 + 2) >> 2);      // X[c]
-    const int e1 = R.lo1 - ((h0 + h1 + 2) >> 2);       // X[c+2]
-    int e2 = __shfl_down_sync(0xFFFFFFFFu, e0, 1);     // X[c+4]
-    if (lane == kLanes - 1) e2 = R.x1 - ((h1 + R.x2 + 2) >> 2);
-    return make_int4(e0, h0 + ((e0 + e1) >> 1), e1, h1 + ((e1 + e2) >> 1));
-  }
-  if (w == 1) return make_int4(R.lo0, 0, 0, 0);
-  const int c = 2 * b;
+// Horizontal lifting of a loaded row: samples of the lane's image columns
+// c .. c+3.  Columns past the right edge return garbage.
+template <bool VEC>
+__device__ __forceinline__ int4 lift_row(const RawRow& R, const Cols& o, int lane) {
+  if (!VEC && o.w == 1) return make_int4(R.lo0, 0, 0, 0);
   int hm1 = __shfl_up_sync(0xFFFFFFFFu, R.hi1, 1);  // X[c-1]
-  if (lane == 0) hm1 = b == 0 ? R.hi0 : R.x1;
-  const int h0 = c + 1 < w ? R.hi0 : hm1;              // X[c+1]
-  const int h1 = c + 3 < w ? R.hi1 : h0;               // X[c+3]
-  const int e0 = R.lo0 - ((hm1 + h0 + 2) >> 2);        // X[c]
-  int e1 = R.lo1 - ((h0 + h1 + 2) >> 2);               // X[c+2]
+  if (lane == 0) hm1 = !VEC || o.left ? R.xh : R.hi0;  // (X[-1] is X[1])
+  const int e0 = R.lo0 - ((hm1 + R.hi0 + 2) >> 2);     // X[c]
+  const int e1 = R.lo1 - ((R.hi0 + R.hi1 + 2) >> 2);   // X[c+2]
   int e2 = __shfl_down_sync(0xFFFFFFFFu, e0, 1);       // X[c+4]
-  if (lane == kLanes - 1 && c + 4 < w) {
-    const int h2 = c + 5 < w ? R.x2 : h1;
-    e2 = R.x1 - ((h1 + h2 + 2) >> 2);
-  }
-  if (c + 2 >= w) e1 = e0;  // column w mirrors column w - 2
-  if (c + 4 >= w) e2 = e1;
-  return make_int4(e0, h0 + ((e0 + e1) >> 1), e1, h1 + ((e1 + e2) >> 1));
-}
-
-template <bool INTERIOR = false>
-__device__ __forceinline__ int4 hrow(const Bands& B, int y, int b, int lane) {
-  return lift_row<INTERIOR>(load_row<INTERIOR>(B, y, b, lane), B.w, b, lane);
+  if (lane == kLanes - 1) e2 = !VEC || o.right ? R.xl - ((R.hi1 + R.xh + 2) >> 2) : e1;  // (X[w] is X[w-2])
+  return make_int4(e0, R.hi0 + ((e0 + e1) >> 1), e1, R.hi1 + ((e1 + e2) >> 1));
 }
 
 __device__ __forceinline__ int4 vupdate(int4 xe, int4 a, int4 c) {
@@ -176,134 +185,65 @@ __device__ __forceinline__ int4 vpredict(int4 xo, int4 a, int4 c) {
 
 // Vertical 5/3 stream over output rows [ys, ye) (ys even) of NC level images
 // at once; emit(y, v[NC]) receives each finished row (four columns per lane).
-// With PREFETCH the loads of row pair m + 1 are issued before row pair m is
-// lifted (more registers; used where a warp streams one component).
-template <int NC, bool PREFETCH, bool INTERIOR, typename Emit>
-__device__ __forceinline__ void stream_rows(const Bands* B, int b, int lane, int ys, int ye, Emit emit) {
-  const int h = B[0].h, w = B[0].w;
+// A component's next row pair is loaded as soon as its registers are free, so
+// the loads of a whole pair are in flight while the current one is lifted and
+// emitted.  What bounds it is the latency of those loads: the lifting state in
+// registers at 16 warps per SM (RGB; 24 with one component) with every load
+// predicated took the last level + pack of the uneven batch from 1.38 to 1.02
+// ms (floor at the copy rate 0.80 ms) and of 256 tiles of 512 x 512 from 0.30
+// to 0.22 ms, against state in shared memory at 32 warps with one component's
+// rows ahead.  Two pairs ahead measured no faster.  tab: the components'
+// bands.
+template <int NC, bool VEC, typename Emit>
+__device__ __forceinline__ void stream_rows(const Bands* tab, const Cols& o, int lane, int ys, int ye, Emit emit) {
+  const int h = o.h;
   int4 v[NC];
   if (h == 1) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) v[c] = hrow<INTERIOR>(B[c], 0, b, lane);
+    for (int c = 0; c < NC; ++c) v[c] = lift_row<VEC>(load_row<VEC>(tab[c].ll, tab[c].hl, 0, o, lane), o, lane);
     emit(0, v);
     return;
   }
+  // Rows -1 .. h + 1 of the symmetric extension (h at least 2).
+  auto row = [&](int y) { return abs(y < h ? y : 2 * (h - 1) - y) >> 1; };
+  // Even rows lie in the low/high pair ll, hl and odd rows in lh, hh;
+  // reflection keeps a row's parity.
+  auto even = [&](int c, int y) { return load_row<VEC>(tab[c].ll, tab[c].hl, row(y), o, lane); };
+  auto odd = [&](int c, int y) { return load_row<VEC>(tab[c].lh, tab[c].hh, row(y), o, lane); };
   int4 xo_prev[NC], ev_prev[NC];
   RawRow re[NC], ro[NC];
+  {
+    RawRow rp[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    re[c] = load_row<INTERIOR>(B[c], ys, b, lane);
-    ro[c] = load_row<INTERIOR>(B[c], ys + 1, b, lane);
-    xo_prev[c] = hrow<INTERIOR>(B[c], ys - 1, b, lane);
-    ev_prev[c] = make_int4(0, 0, 0, 0);
-  }
-  for (int m = ys >> 1;; ++m) {
-    const int ye_row = 2 * m, yo_row = 2 * m + 1;
-    const bool more = yo_row < ye;
-    const bool first = m == (ys >> 1);
-    RawRow ne[NC], no[NC];
-    int4 ev[NC], xo[NC];
+    for (int c = 0; c < NC; ++c) rp[c] = odd(c, ys - 1);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      // Without PREFETCH one component's rows are loaded at a time.
-      if (!PREFETCH && !first) {
-        re[c] = load_row<INTERIOR>(B[c], ye_row, b, lane);
-        ro[c] = load_row<INTERIOR>(B[c], yo_row, b, lane);
-      }
-      if (PREFETCH && more) {
-        ne[c] = load_row<INTERIOR>(B[c], ye_row + 2, b, lane);
-        no[c] = load_row<INTERIOR>(B[c], yo_row + 2, b, lane);
-      }
-      const int4 xe = lift_row<INTERIOR>(re[c], w, b, lane);
-      xo[c] = lift_row<INTERIOR>(ro[c], w, b, lane);
-      ev[c] = vupdate(xe, xo_prev[c], xo[c]);
+      re[c] = even(c, ys);
+      ro[c] = odd(c, ys + 1);
     }
-    if (ye_row - 1 >= ys && ye_row - 1 < ye) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) v[c] = vpredict(xo_prev[c], ev_prev[c], ev[c]);
-      emit(ye_row - 1, v);
-    }
-    if (ye_row < ye) emit(ye_row, ev);
-    if (!more) break;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      xo_prev[c] = xo[c];
-      ev_prev[c] = ev[c];
-      if (PREFETCH) {
-        re[c] = ne[c];
-        ro[c] = no[c];
+      xo_prev[c] = lift_row<VEC>(rp[c], o, lane);
+      ev_prev[c] = make_int4(0, 0, 0, 0);
+    }
+  }
+  for (int y = ys;; y += 2) {
+    const bool more = y + 1 < ye;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int4 xe = lift_row<VEC>(re[c], o, lane), xo = lift_row<VEC>(ro[c], o, lane);
+      if (more) {
+        re[c] = even(c, y + 2);
+        ro[c] = odd(c, y + 3);
       }
+      const int4 ev = vupdate(xe, xo_prev[c], xo);
+      v[c] = vpredict(xo_prev[c], ev_prev[c], ev);
+      xo_prev[c] = xo;
+      ev_prev[c] = ev;
     }
-  }
-}
-
-// Per-lane shared-memory slots (int4 each) of the three-component stream:
-// 0..2 previous odd row (horizontally lifted), 3..5 previous updated even
-// row (also the finished row 2m), 6..8 the finished row 2m - 1.
-constexpr int kStreamSlots = 9;
-
-// Vertical 5/3 stream over rows [ys, ye) of three level images, one
-// component at a time: the lifting state lives in the lane's own
-// shared-memory slots `st` (slot k at st[k * 32 + lane]) and the components'
-// band descriptors in the warp's shared table `tab`, so only one
-// component's rows are in registers at once.  emit(y, v[3]) as stream_rows.
-template <bool INTERIOR, typename Emit>
-__device__ __forceinline__ void stream_rows3(const Bands* tab, int b, int lane, int ys, int ye, int4* st,
-                                             Emit emit) {
-  const int w = tab[0].w, h = tab[0].h;
-  auto bands = [&](int c) -> const Bands& { return tab[c]; };
-  auto slot = [&](int k) -> int4& { return st[k * kLanes + lane]; };
-  int4 v[3];
-  if (h == 1) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) v[c] = hrow<INTERIOR>(bands(c), 0, b, lane);
-    emit(0, v);
-    return;
-  }
-#pragma unroll 1
-  for (int c = 0; c < 3; ++c) {
-    slot(c) = hrow<INTERIOR>(bands(c), ys - 1, b, lane);
-    slot(3 + c) = make_int4(0, 0, 0, 0);
-  }
-  // The rows of the next component (or of the next row pair's first
-  // component) are loaded while the current one is lifted.
-  RawRow re = load_row<INTERIOR>(bands(0), ys, b, lane), ro = load_row<INTERIOR>(bands(0), ys + 1, b, lane);
-  for (int m = ys >> 1;; ++m) {
-    const int ye_row = 2 * m, yo_row = 2 * m + 1;
-    const bool more = yo_row < ye;
-#pragma unroll 1
-    for (int c = 0; c < 3; ++c) {
-      RawRow ne = re, no = ro;
-      if (c < 2) {
-        const Bands& N = bands(c + 1);
-        ne = load_row<INTERIOR>(N, ye_row, b, lane);
-        no = load_row<INTERIOR>(N, yo_row, b, lane);
-      } else if (more) {
-        const Bands& N = bands(0);
-        ne = load_row<INTERIOR>(N, ye_row + 2, b, lane);
-        no = load_row<INTERIOR>(N, yo_row + 2, b, lane);
-      }
-      const int4 xe = lift_row<INTERIOR>(re, w, b, lane);
-      const int4 xo = lift_row<INTERIOR>(ro, w, b, lane);
-      re = ne;
-      ro = no;
-      const int4 xo_prev = slot(c), ev_prev = slot(3 + c);
-      const int4 ev = vupdate(xe, xo_prev, xo);
-      slot(6 + c) = vpredict(xo_prev, ev_prev, ev);
-      slot(c) = xo;
-      slot(3 + c) = ev;
-    }
-    if (ye_row - 1 >= ys && ye_row - 1 < ye) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) v[c] = slot(6 + c);
-      emit(ye_row - 1, v);
-    }
-    if (ye_row < ye) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) v[c] = slot(3 + c);
-      emit(ye_row, v);
-    }
-    if (yo_row >= ye) break;
+    if (y > ys) emit(y - 1, v);
+    if (y < ye) emit(y, ev_prev);
+    if (!more) return;
   }
 }
 
@@ -346,8 +286,8 @@ __device__ __forceinline__ void idwt_unit(const IdwtJob* __restrict__ jobs, uint
   const int ys = (int)job.y_begin + (int)(local / job.strips) * (int)job.seg;
   const int w = (int)job.w, h = (int)job.h;
   const int ye = min(ys + (int)job.seg, (int)job.y_end);
-  const Bands B = make_bands(job.ll, job.hl, job.lh, job.hh, w, h);
-  const int b = (x0 >> 1) + 2 * lane, col = 2 * b;
+  const Bands B{job.ll, job.hl, job.lh, job.hh};
+  const int col = x0 + 4 * lane;
   int32_t* out = job.out;
   // Rows of w int32 from a 16-byte aligned base: 16-byte stores when w % 4 == 0.
   const bool vec_out = (w & 3) == 0 && (((uintptr_t)out) & 15) == 0;
@@ -362,8 +302,10 @@ __device__ __forceinline__ void idwt_unit(const IdwtJob* __restrict__ jobs, uint
       if (col + 3 < w) row[col + 3] = v[0].w;
     }
   };
-  if (interior_strip(x0, w)) stream_rows<1, true, true>(&B, b, lane, ys, ye, emit);
-  else stream_rows<1, true, false>(&B, b, lane, ys, ye, emit);
+  if (x0 + kIdwtStripW <= w && aligned_bands(B, w))
+    stream_rows<1, true>(&B, make_cols<true>(x0, w, h, lane), lane, ys, ye, emit);
+  else
+    stream_rows<1, false>(&B, make_cols<false>(x0, w, h, lane), lane, ys, ye, emit);
 }
 
 }  // namespace
@@ -432,6 +374,19 @@ __host__ __device__ constexpr int pack_bpp() {
 
 // Byte q (a compile-time constant after unrolling) of a lane's packed words.
 __device__ __forceinline__ void put_byte(uint32_t* wds, int q, uint32_t byte) { wds[q >> 2] |= byte << (8 * (q & 3)); }
+
+// Four samples clamped to [0, 255], the first in the low byte.
+__device__ __forceinline__ uint32_t pack_u8x4(int32_t a, int32_t b, int32_t c, int32_t d) {
+#ifdef __CUDA_ARCH__
+  uint32_t hi, r;
+  asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(d), "r"(c), "r"(0));
+  asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(b), "r"(a), "r"(hi));
+  return r;
+#else
+  auto u = [](int32_t v) { return (uint32_t)min(max(v, 0), 255); };
+  return u(a) | (u(b) << 8) | (u(c) << 16) | (u(d) << 24);
+#endif
+}
 
 // Packs pixel p (components c0..c2 after the inverse RCT and DC shift) at
 // byte p * bpp of the lane's four-pixel group.
@@ -517,56 +472,73 @@ __device__ __forceinline__ void store_row(uint8_t* g, int x0, int xs, int nbytes
 
 template <int NC, int FMT, bool DIRECT>
 __device__ __forceinline__ void pack_unit(const PackJob& job, int x0, int ys, int ye, int lane, uint32_t* rowbuf,
-                                          int4* st, Bands* tab) {
+                                          Bands* tab) {
   constexpr int BPP = pack_bpp<FMT>();
   const int w = (int)job.w;
   const int cx0 = (int)job.cx, cy0 = (int)job.cy, cx1 = cx0 + (int)job.cw, cy1 = cy0 + (int)job.ch;
   const uint32_t bd = job.bit_depth, reg = job.region_conv;
   const int32_t shift = 1 << (bd - 1);
   const bool mct = NC == 3 && job.mct;
-  const int b = (x0 >> 1) + 2 * lane, col = 2 * b;
+  const int col = x0 + 4 * lane;
   const int xs = max(x0, cx0), xe = min(x0 + kIdwtStripW, cx1);
   const int nbytes = (xe - xs) * BPP;
+  uint8_t* const first = job.out + (uint64_t)(xs - cx0) * BPP;
+  const uint64_t pitch = job.pitch;
   auto emit = [&](int y, const int4* v) {
     if (y < cy0 || y >= cy1) return;  // warp-uniform
-    uint32_t wds[BPP];
-#pragma unroll
-    for (int k = 0; k < BPP; ++k) wds[k] = 0;
+    // The DC shift joins the luma before the inverse RCT, whose other two
+    // components are sums with the green that comes out of it.
+    int32_t px[4][NC];
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-      int32_t c0 = lane_comp(v[0], p), c1 = 0, c2 = 0;
+      px[p][0] = lane_comp(v[0], p) + shift;
       if (NC == 3) {
-        c1 = lane_comp(v[1], p);
-        c2 = lane_comp(v[2], p);
+        const int32_t c1 = lane_comp(v[1], p), c2 = lane_comp(v[2], p);
         if (mct) {
-          const int32_t gg = c0 - ((c2 + c1) >> 2);
-          const int32_t r = c2 + gg, bl = c1 + gg;
-          c0 = r;
-          c1 = gg;
-          c2 = bl;
+          const int32_t g = px[p][0] - ((c2 + c1) >> 2);
+          px[p][0] = c2 + g;
+          px[p][1] = g;
+          px[p][2] = c1 + g;
+        } else {
+          px[p][1] = c1 + shift;
+          px[p][2] = c2 + shift;
         }
-        c1 += shift;
-        c2 += shift;
       }
-      c0 += shift;
-      put_pixel<FMT, DIRECT>(wds, p, c0, c1, c2, bd, reg);
     }
-    store_row<BPP>(job.out + (uint64_t)(y - cy0) * job.pitch + (uint64_t)(xs - cx0) * BPP, x0, xs, nbytes, lane,
-                   rowbuf, wds);
+    uint32_t wds[BPP];
+    if constexpr (DIRECT && FMT == PACK_GRAY8) {
+      wds[0] = pack_u8x4(px[0][0], px[1][0], px[2][0], px[3][0]);
+    } else if constexpr (DIRECT && FMT == PACK_RGB8) {
+      wds[0] = pack_u8x4(px[0][0], px[0][1], px[0][2], px[1][0]);
+      wds[1] = pack_u8x4(px[1][1], px[1][2], px[2][0], px[2][1]);
+      wds[2] = pack_u8x4(px[2][2], px[3][0], px[3][1], px[3][2]);
+    } else if constexpr (DIRECT && FMT == PACK_RGBA8) {
+#pragma unroll
+      for (int p = 0; p < 4; ++p) wds[p] = pack_u8x4(px[p][0], px[p][1], px[p][2], 255);
+    } else {
+#pragma unroll
+      for (int k = 0; k < BPP; ++k) wds[k] = 0;
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+        put_pixel<FMT, DIRECT>(wds, p, px[p][0], px[p][NC == 3 ? 1 : 0], px[p][NC == 3 ? 2 : 0], bd, reg);
+    }
+    store_row<BPP>(first + (uint64_t)(y - cy0) * pitch, x0, xs, nbytes, lane, rowbuf, wds);
   };
   if (job.lifting) {
+    // The components' band descriptors: read from the job once per unit into
+    // the warp's shared table (RGB), or in registers (gray).
+    const int h = (int)job.h;
+    Bands one{job.ll[0], job.hl[0], job.lh[0], job.hh[0]};
+    bool vec = x0 + kIdwtStripW <= w && aligned_bands(one, w);
     if (NC == 3) {
-      // The components' band descriptors, read from the job once per unit.
-      if (lane < 3) tab[lane] = make_bands(job.ll[lane], job.hl[lane], job.lh[lane], job.hh[lane], w, (int)job.h);
+      for (int c = 1; c < 3; ++c) vec = vec && aligned_bands(Bands{job.ll[c], job.hl[c], job.lh[c], job.hh[c]}, w);
+      if (lane < 3) tab[lane] = Bands{job.ll[lane], job.hl[lane], job.lh[lane], job.hh[lane]};
       __syncwarp();
-      if (interior_strip(x0, w)) stream_rows3<true>(tab, b, lane, ys, ye, st, emit);
-      else stream_rows3<false>(tab, b, lane, ys, ye, st, emit);
-      __syncwarp();  // the table is rewritten by the warp's next unit
-    } else {
-      const Bands B = make_bands(job.ll[0], job.hl[0], job.lh[0], job.hh[0], w, (int)job.h);
-      if (interior_strip(x0, w)) stream_rows<1, true, true>(&B, b, lane, ys, ye, emit);
-      else stream_rows<1, true, false>(&B, b, lane, ys, ye, emit);
     }
+    const Bands* B = NC == 3 ? tab : &one;
+    if (vec) stream_rows<NC, true>(B, make_cols<true>(x0, w, h, lane), lane, ys, ye, emit);
+    else stream_rows<NC, false>(B, make_cols<false>(x0, w, h, lane), lane, ys, ye, emit);
+    if (NC == 3) __syncwarp();  // the table is rewritten by the warp's next unit
   } else {
     // Nothing left to lift: the image is the LL band itself.
     for (int y = ys; y < ye; ++y) {
@@ -588,39 +560,35 @@ __device__ __forceinline__ void pack_unit(const PackJob& job, int x0, int ys, in
 
 template <int FMT, int NC, bool DIRECT>
 __device__ __forceinline__ void pack_one(const PackJob* __restrict__ jobs, uint32_t njobs, uint32_t unit,
-                                         uint32_t* rowbuf, int4* st, Bands* tab) {
+                                         uint32_t* rowbuf, Bands* tab) {
   const int lane = threadIdx.x & 31;
   const PackJob& job = find_job(jobs, njobs, unit);
   const uint32_t local = unit - job.unit_begin;
   const int x0 = (int)(job.cx & ~(uint32_t)(kIdwtStripW - 1)) + (int)(local % job.strips) * kIdwtStripW;
   const int ys = (int)(job.cy & ~1u) + (int)(local / job.strips) * (int)job.seg;
   const int ye = min(ys + (int)job.seg, (int)(job.cy + job.ch));
-  pack_unit<NC, FMT, DIRECT>(job, x0, ys, ye, lane, rowbuf, st, tab);
+  pack_unit<NC, FMT, DIRECT>(job, x0, ys, ye, lane, rowbuf, tab);
 }
 
 // One kernel per (pixel format, components, conversion) variant, with the
 // jobs of a launch all of that variant (pack_variant): each variant gets the
 // registers it needs and none of the others' code.  NC 3: RGB tiles, 1: gray;
-// DIRECT: samples convert with a clamp alone.  The gray stream keeps its
-// lifting state in registers (the RGB one in shared memory), so it runs
-// three CTAs per SM with room for it instead of four.
+// DIRECT: samples convert with a clamp alone.
 template <int FMT, int NC, bool DIRECT, bool QUEUE>
-__global__ void __launch_bounds__(kIdwtWarps * 32, NC == 3 ? 4 : 3) pack_kernel(const PackJob* __restrict__ jobs, uint32_t njobs,
+__global__ void __launch_bounds__(kIdwtWarps * 32, NC == 3 ? 2 : 3) pack_kernel(const PackJob* __restrict__ jobs, uint32_t njobs,
                                                                uint32_t nunits, uint32_t* queue) {
   __shared__ __align__(16) uint32_t rowbufs[kIdwtWarps][kRowWords];
-  __shared__ int4 states[kIdwtWarps][kStreamSlots * kLanes];
   __shared__ Bands tabs[kIdwtWarps][3];
   uint32_t* rowbuf = rowbufs[threadIdx.x >> 5];
-  int4* st = states[threadIdx.x >> 5];
   Bands* tab = tabs[threadIdx.x >> 5];
   if (!QUEUE) {
     const uint32_t unit = blockIdx.x * kIdwtWarps + (threadIdx.x >> 5);
-    if (unit < nunits) pack_one<FMT, NC, DIRECT>(jobs, njobs, unit, rowbuf, st, tab);
+    if (unit < nunits) pack_one<FMT, NC, DIRECT>(jobs, njobs, unit, rowbuf, tab);
     return;
   }
   bool first = true;
   for (uint32_t unit; next_unit(queue, nunits, first, unit);)
-    pack_one<FMT, NC, DIRECT>(jobs, njobs, unit, rowbuf, st, tab);
+    pack_one<FMT, NC, DIRECT>(jobs, njobs, unit, rowbuf, tab);
 }
 
 // ---------------------------------------------------------------------------
@@ -657,21 +625,6 @@ static_assert(kStrip97 == 4 * (kLanes - 2), "lanes 1..30 hold a strip's output c
 
 namespace {
 
-// Whole-sample symmetric extension into [0, n) of an index at most four
-// samples outside it (every sample an exact output depends on).  Indices
-// further out (columns of lanes whose results are unused) end at the nearest
-// in-range index of the same parity, so the band they select (low for even,
-// high for odd) and the row inside it stay in bounds.
-__device__ __forceinline__ int fold97(int i, int n) {
-  if ((unsigned)i < (unsigned)n) return i;
-  if (n == 1) return 0;
-#pragma unroll 1
-  for (int k = 0; k < 4 && (unsigned)i >= (unsigned)n; ++k) i = i < 0 ? -i : 2 * (n - 1) - i;
-  if (i < 0) return i & 1;
-  if (i >= n) return (n - 1) - (((n - 1) ^ i) & 1);
-  return i;
-}
-
 struct Src97 {
   const int32_t* ll;
   const int32_t* hl;
@@ -697,7 +650,7 @@ struct Raw97 {
 };
 
 __device__ __forceinline__ void row_bands(const Src97& S, int y, const int32_t*& lo, const int32_t*& hi) {
-  y = fold97(y, S.h);
+  y = reflect(y, S.h);
   const int r = y >> 1;
   lo = ((y & 1) ? S.lh : S.ll) + (size_t)r * ((S.w + 1) >> 1);
   hi = ((y & 1) ? S.hh : S.hl) + (size_t)r * (S.w >> 1);
@@ -714,8 +667,8 @@ __device__ __forceinline__ Raw97 load97(const Src97& S, int y, int c) {
   }
   // Reflection keeps a column's parity, so even columns stay in the low band.
   const int w = S.w;
-  return Raw97{__ldg(lo + (fold97(c, w) >> 1)), __ldg(hi + (fold97(c + 1, w) >> 1)), __ldg(lo + (fold97(c + 2, w) >> 1)),
-               __ldg(hi + (fold97(c + 3, w) >> 1))};
+  return Raw97{__ldg(lo + (reflect(c, w) >> 1)), __ldg(hi + (reflect(c + 1, w) >> 1)), __ldg(lo + (reflect(c + 2, w) >> 1)),
+               __ldg(hi + (reflect(c + 3, w) >> 1))};
 }
 
 __device__ __forceinline__ float lstep(float l, float r, float c, float x) { return fmaf(__fadd_rn(l, r), c, x); }
@@ -723,7 +676,7 @@ __device__ __forceinline__ float lstep(float l, float r, float c, float x) { ret
 // Dequantises (or reinterprets) a loaded row and runs the horizontal 9/7
 // synthesis: the lane's four columns (exact on lanes 1..30).
 __device__ __forceinline__ float4 lift97(const Src97& S, int y, const Raw97& R, float K, float IK) {
-  const bool odd = fold97(y, S.h) & 1;
+  const bool odd = reflect(y, S.h) & 1;
   const float ql = odd ? S.q[2] : S.q[0], qh = odd ? S.q[3] : S.q[1];
   float e0, e1;
   if (!odd && !S.ll_band) {
