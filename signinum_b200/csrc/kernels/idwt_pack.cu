@@ -30,6 +30,7 @@
 // the warp's row buffer where the row does not fall on lane boundaries.
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 
 #include "../device_plan.h"
 #include "kernels.h"
@@ -615,12 +616,18 @@ __global__ void __launch_bounds__(kIdwtWarps * 32, NC == 3 ? 2 : 3) pack_kernel(
 // lanes' own results are not used).  Vertically a four-stage pipeline runs
 // down the rows, loading rows 2m+2 and 2m+3 per step and finishing rows 2m
 // (after beta) and 2m-1 (after alpha); a unit starting at row ys primes from
-// row ys-3.  The next rows' raw samples are loaded one step (or, for three
-// components, one component) ahead.
+// row ys-3.  The lifting state sits in registers, a lane's column offsets are
+// reflected once per unit, and a component's next rows load as soon as its
+// registers are free.  What bounds it: the latency of the dependent f32 steps
+// at 12 warps per SM.  128 tiles of 512 x 512 RGB: levels 0.36 -> 0.15 ms and
+// last level + ICT + pack 0.59 -> 0.24 ms, against lifting state in shared
+// memory and columns reflected per row; four CTAs per SM (128 registers, 90
+// bytes of spills) 0.26 ms; the pack with every bit depth's conversion in one
+// loop 0.54 ms.
 
 constexpr float kNegAlpha97 = 1.5861343f, kNegBeta97 = 0.052980117f, kNegGamma97 = -0.8829111f,
                 kNegDelta97 = -0.44350687f, kKappa97 = 1.2301741f;
-constexpr int kWarps97 = 4;  // warps per CTA of the 9/7 pack kernel (its shared state is larger)
+constexpr int kWarps97 = 4;  // warps per CTA of the 9/7 pack kernel
 static_assert(kStrip97 == 4 * (kLanes - 2), "lanes 1..30 hold a strip's output columns");
 
 namespace {
@@ -630,17 +637,27 @@ struct Src97 {
   const int32_t* hl;
   const int32_t* lh;
   const int32_t* hh;
-  float q[4];    // dequantisation steps of ll, hl, lh, hh
-  int w, h;
-  bool ll_band;  // ll is the LL band; otherwise the previous level's f32 image
-  bool fast;     // the strip's 128 columns lie inside the level and rows are 8-byte aligned
+  float q[4];  // dequantisation steps of ll, hl, lh, hh
 };
 
-__device__ __forceinline__ Src97 make_src97(const int32_t* ll, const int32_t* hl, const int32_t* lh,
-                                            const int32_t* hh, const float* q, bool ll_band, int w, int h, int c0) {
-  const uintptr_t a = (uintptr_t)ll | (uintptr_t)hl | (uintptr_t)lh | (uintptr_t)hh;
-  const bool fast = (w & 3) == 0 && (a & 7) == 0 && c0 >= 0 && c0 + 4 * kLanes <= w;
-  return Src97{ll, hl, lh, hh, {q[0], q[1], q[2], q[3]}, w, h, ll_band, fast};
+// A lane's columns: band offsets of its image columns c .. c+3 (low band l0,
+// l1; high band h0, h1).  VEC: the strip's 128 columns lie inside the level
+// and its rows are 8-byte aligned, so each band's pair is one load.
+struct Cols97 {
+  int w, h;
+  int l0, l1, h0, h1;
+  bool ll_band;  // ll is the LL band; otherwise the previous level's f32 image
+};
+
+__device__ __forceinline__ bool vec97(const Src97& S, int w, int c0) {
+  const uintptr_t a = (uintptr_t)S.ll | (uintptr_t)S.hl | (uintptr_t)S.lh | (uintptr_t)S.hh;
+  return (w & 3) == 0 && (a & 7) == 0 && c0 >= 0 && c0 + 4 * kLanes <= w;
+}
+
+template <bool VEC>
+__device__ __forceinline__ Cols97 make_cols97(int c, int w, int h, bool ll_band) {
+  if (VEC) return Cols97{w, h, c >> 1, 0, c >> 1, 0, ll_band};
+  return Cols97{w, h, reflect(c, w) >> 1, reflect(c + 2, w) >> 1, reflect(c + 1, w) >> 1, reflect(c + 3, w) >> 1, ll_band};
 }
 
 // The raw words of a lane's four columns of one interleaved row (low band at
@@ -649,45 +666,30 @@ struct Raw97 {
   int32_t e0, o0, e1, o1;
 };
 
-__device__ __forceinline__ void row_bands(const Src97& S, int y, const int32_t*& lo, const int32_t*& hi) {
-  y = reflect(y, S.h);
-  const int r = y >> 1;
-  lo = ((y & 1) ? S.lh : S.ll) + (size_t)r * ((S.w + 1) >> 1);
-  hi = ((y & 1) ? S.hh : S.hl) + (size_t)r * (S.w >> 1);
-}
-
-// c: the lane's first column (even).
-__device__ __forceinline__ Raw97 load97(const Src97& S, int y, int c) {
-  const int32_t *lo, *hi;
-  row_bands(S, y, lo, hi);
-  if (S.fast) {
-    const int2 l = __ldg(reinterpret_cast<const int2*>(lo + (c >> 1)));
-    const int2 h = __ldg(reinterpret_cast<const int2*>(hi + (c >> 1)));
+// Row r of the low and the high band.
+template <bool VEC>
+__device__ __forceinline__ Raw97 load97(const int32_t* low, const int32_t* high, int r, const Cols97& o) {
+  const int32_t* lo = low + (size_t)r * ((o.w + 1) >> 1) + o.l0;
+  const int32_t* hi = high + (size_t)r * (o.w >> 1) + o.h0;
+  if (VEC) {
+    const int2 l = __ldg(reinterpret_cast<const int2*>(lo));
+    const int2 h = __ldg(reinterpret_cast<const int2*>(hi));
     return Raw97{l.x, h.x, l.y, h.y};
   }
-  // Reflection keeps a column's parity, so even columns stay in the low band.
-  const int w = S.w;
-  return Raw97{__ldg(lo + (reflect(c, w) >> 1)), __ldg(hi + (reflect(c + 1, w) >> 1)), __ldg(lo + (reflect(c + 2, w) >> 1)),
-               __ldg(hi + (reflect(c + 3, w) >> 1))};
+  const bool high_band = o.w > 1;  // a single column has none
+  return Raw97{__ldg(lo), load_if(high_band, hi), __ldg(lo + (o.l1 - o.l0)), load_if(high_band, hi + (o.h1 - o.h0))};
 }
 
 __device__ __forceinline__ float lstep(float l, float r, float c, float x) { return fmaf(__fadd_rn(l, r), c, x); }
 
 // Dequantises (or reinterprets) a loaded row and runs the horizontal 9/7
-// synthesis: the lane's four columns (exact on lanes 1..30).
-__device__ __forceinline__ float4 lift97(const Src97& S, int y, const Raw97& R, float K, float IK) {
-  const bool odd = reflect(y, S.h) & 1;
-  const float ql = odd ? S.q[2] : S.q[0], qh = odd ? S.q[3] : S.q[1];
-  float e0, e1;
-  if (!odd && !S.ll_band) {
-    e0 = __int_as_float(R.e0);
-    e1 = __int_as_float(R.e1);
-  } else {
-    e0 = __fmul_rn(__int2float_rn(R.e0), ql);
-    e1 = __fmul_rn(__int2float_rn(R.e1), ql);
-  }
+// synthesis: the lane's four columns (exact on lanes 1..30).  IMAGE: the low
+// band's words are the previous level's f32 samples.
+__device__ __forceinline__ float4 lift97(const Raw97& R, float ql, float qh, bool image, bool single, float K, float IK) {
+  float e0 = image ? __int_as_float(R.e0) : __fmul_rn(__int2float_rn(R.e0), ql);
+  float e1 = image ? __int_as_float(R.e1) : __fmul_rn(__int2float_rn(R.e1), ql);
   float o0 = __fmul_rn(__int2float_rn(R.o0), qh), o1 = __fmul_rn(__int2float_rn(R.o1), qh);
-  if (S.w == 1) return make_float4(e0, 0.0f, 0.0f, 0.0f);
+  if (single) return make_float4(e0, 0.0f, 0.0f, 0.0f);
   e0 = __fmul_rn(e0, K);
   e1 = __fmul_rn(e1, K);
   o0 = __fmul_rn(o0, IK);
@@ -711,87 +713,74 @@ __device__ __forceinline__ float4 lstep4(float4 a, float4 b, float c, float4 x) 
                      lstep(a.w, b.w, c, x.w));
 }
 
-// Vertical 9/7 stream over rows [ys, ye) (ys even) of NC level images.
-// col is the lane's first column; src(c) gives component c's bands;
-// st(c, k) is its lifting state (k 0: the
-// last odd input row, 1..3: the last rows after delta, gamma, beta, the
-// beta row being the step's finished even row; 4: its finished odd row);
-// emit(y, v[NC]) receives each
-// finished row.  Components are lifted one at a time while the next
-// component's (or the next step's) rows load.
-template <int NC, typename SrcOf, typename State, typename Emit>
-__device__ __forceinline__ void stream97(SrcOf src, int h, int col, int ys, int ye, float K, float IK, State st,
+// Vertical 9/7 stream over rows [ys, ye) (ys even) of NC level images, one
+// component after the other; emit(y, v[NC]) receives each finished row.
+template <int NC, bool VEC, typename Emit>
+__device__ __forceinline__ void stream97(const Src97* tab, const Cols97& o, int ys, int ye, float K, float IK,
                                          Emit emit) {
+  const int h = o.h;
+  const bool image = !o.ll_band, single = !VEC && o.w == 1;
   float4 v[NC];
+  auto even97 = [&](int c, const Raw97& R) { return lift97(R, tab[c].q[0], tab[c].q[1], image, single, K, IK); };
+  auto odd97 = [&](int c, const Raw97& R) { return lift97(R, tab[c].q[2], tab[c].q[3], false, single, K, IK); };
   if (h == 1) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const Src97& S = src(c);
-      v[c] = lift97(S, 0, load97(S, 0, col), K, IK);
-    }
+    for (int c = 0; c < NC; ++c) v[c] = even97(c, load97<VEC>(tab[c].ll, tab[c].hl, 0, o));
     emit(0, v);
     return;
   }
-  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 1
-  for (int c = 0; c < NC; ++c) {
-    const Src97& S = src(c);
-    st(c, 0) = scale4(lift97(S, ys - 3, load97(S, ys - 3, col), K, IK), IK);
-    st(c, 1) = zero;
-    st(c, 2) = zero;
-    st(c, 3) = zero;
-  }
-  const int m0 = (ys >> 1) - 2, m1 = ye >> 1;
-  Raw97 re, ro;
+  // Rows -4 .. h + 3 of the symmetric extension (h at least 2; rows that no
+  // finished row depends on may be asked for further out when h is 2).
+  auto row = [&](int y) {
+    int t = abs(y);
+    t = t < h ? t : abs(2 * (h - 1) - t);
+    t = t < h ? t : abs(2 * (h - 1) - t);
+    return (t < h ? t : t & 1) >> 1;
+  };
+  auto even = [&](int c, int y) { return load97<VEC>(tab[c].ll, tab[c].hl, row(y), o); };
+  auto odd = [&](int c, int y) { return load97<VEC>(tab[c].lh, tab[c].hh, row(y), o); };
+  const int y1 = ye & ~1;  // the last step's even row
+  int y = ys - 4;          // the step's even row: rows y + 2, y + 3 come in
+  // Per component: the last odd row in, the last rows after delta and gamma,
+  // and the last finished even row.
+  float4 xp[NC], s1p[NC], s2p[NC], s3p[NC];
+  Raw97 re[NC], ro[NC];
   {
-    const Src97& S = src(0);
-    re = load97(S, 2 * m0 + 2, col);
-    ro = load97(S, 2 * m0 + 3, col);
-  }
-  for (int m = m0; m <= m1; ++m) {
-#pragma unroll 1
-    for (int c = 0; c < NC; ++c) {
-      // Loads of the next component's rows, or of the next step's first one.
-      Raw97 ne = re, no = ro;
-      if (c + 1 < NC) {
-        const Src97& N = src(c + 1);
-        ne = load97(N, 2 * m + 2, col);
-        no = load97(N, 2 * m + 3, col);
-      } else if (m < m1) {
-        const Src97& N = src(0);
-        ne = load97(N, 2 * m + 4, col);
-        no = load97(N, 2 * m + 5, col);
-      }
-      const Src97& S = src(c);
-      const float4 xe = scale4(lift97(S, 2 * m + 2, re, K, IK), K);
-      const float4 xo = scale4(lift97(S, 2 * m + 3, ro, K, IK), IK);
-      re = ne;
-      ro = no;
-      const float4 xp = st(c, 0), s1p = st(c, 1), s2p = st(c, 2), s3p = st(c, 3);
-      const float4 s1 = lstep4(xp, xo, kNegDelta97, xe);   // row 2m+2
-      const float4 s2 = lstep4(s1p, s1, kNegGamma97, xp);  // row 2m+1
-      const float4 s3 = lstep4(s2p, s2, kNegBeta97, s1p);  // row 2m, final
-      st(c, 4) = lstep4(s3p, s3, kNegAlpha97, s2p);        // row 2m-1, final
-      st(c, 0) = xo;
-      st(c, 1) = s1;
-      st(c, 2) = s2;
-      st(c, 3) = s3;
-    }
-    // The step's finished odd row 2m - 1, then its even row 2m, through one
-    // call site of emit (its pixel conversions are long: one copy of them
-    // in the loop keeps the code small).
-#pragma unroll 1
-    for (int k = 0; k < 2; ++k) {
-      const int y = 2 * m - 1 + k;
-      if (y >= ys && y < ye) {
+    Raw97 rp[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const float4 odd = st(c, 4), even = st(c, 3);
-          v[c] = k ? even : odd;
-        }
-        emit(y, v);
-      }
+    for (int c = 0; c < NC; ++c) rp[c] = odd(c, ys - 3);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      re[c] = even(c, y + 2);
+      ro[c] = odd(c, y + 3);
     }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      xp[c] = scale4(odd97(c, rp[c]), IK);
+      s1p[c] = s2p[c] = s3p[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+  }
+  for (;; y += 2) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const float4 xe = scale4(even97(c, re[c]), K);
+      const float4 xo = scale4(odd97(c, ro[c]), IK);
+      if (y < y1) {
+        re[c] = even(c, y + 4);
+        ro[c] = odd(c, y + 5);
+      }
+      const float4 s1 = lstep4(xp[c], xo, kNegDelta97, xe);   // row y + 2
+      const float4 s2 = lstep4(s1p[c], s1, kNegGamma97, xp[c]);  // row y + 1
+      const float4 s3 = lstep4(s2p[c], s2, kNegBeta97, s1p[c]);  // row y, final
+      v[c] = lstep4(s3p[c], s3, kNegAlpha97, s2p[c]);            // row y - 1, final
+      xp[c] = xo;
+      s1p[c] = s1;
+      s2p[c] = s2;
+      s3p[c] = s3;
+    }
+    if (y > ys) emit(y - 1, v);
+    if (y >= ys && y < ye) emit(y, s3p);
+    if (y >= y1) return;
   }
 }
 
@@ -804,26 +793,25 @@ __device__ __forceinline__ void idwt97_unit(const IdwtJob* __restrict__ jobs, ui
   const int w = (int)job.w, h = (int)job.h;
   const int ye = min(ys + (int)job.seg, (int)job.y_end);
   const int col = x0 - 4 + 4 * lane;
-  const Src97 S = make_src97(job.ll, job.hl, job.lh, job.hh, job.step, job.ll_band != 0, w, h, x0 - 4);
+  const Src97 S{job.ll, job.hl, job.lh, job.hh, {job.step[0], job.step[1], job.step[2], job.step[3]}};
   float* out = reinterpret_cast<float*>(job.out);
   const bool mine = lane >= 1 && lane <= kLanes - 2;
   const bool vec_out = (w & 3) == 0 && (((uintptr_t)out) & 15) == 0;
-  float4 state[5];
-  const Src97* sp = &S;
-  stream97<1>([sp](int) -> const Src97& { return *sp; }, h, col, ys, ye, kKappa97, IK,
-              [&](int, int k) -> float4& { return state[k]; },
-              [&](int y, const float4* v) {
-                if (!mine) return;
-                float* rowp = out + (size_t)y * w;
-                if (vec_out && col + 3 < w) {
-                  *reinterpret_cast<float4*>(rowp + col) = v[0];
-                } else {
-                  if (col < w) rowp[col] = v[0].x;
-                  if (col + 1 < w) rowp[col + 1] = v[0].y;
-                  if (col + 2 < w) rowp[col + 2] = v[0].z;
-                  if (col + 3 < w) rowp[col + 3] = v[0].w;
-                }
-              });
+  const bool ll_band = job.ll_band != 0;
+  auto emit = [&](int y, const float4* v) {
+    if (!mine) return;
+    float* rowp = out + (size_t)y * w;
+    if (vec_out && col + 3 < w) {
+      *reinterpret_cast<float4*>(rowp + col) = v[0];
+    } else {
+      if (col < w) rowp[col] = v[0].x;
+      if (col + 1 < w) rowp[col + 1] = v[0].y;
+      if (col + 2 < w) rowp[col + 2] = v[0].z;
+      if (col + 3 < w) rowp[col + 3] = v[0].w;
+    }
+  };
+  if (vec97(S, w, x0 - 4)) stream97<1, true>(&S, make_cols97<true>(col, w, h, ll_band), ys, ye, kKappa97, IK, emit);
+  else stream97<1, false>(&S, make_cols97<false>(col, w, h, ll_band), ys, ye, kKappa97, IK, emit);
 }
 
 }  // namespace
@@ -855,19 +843,36 @@ __device__ __forceinline__ uint32_t sat_u8_round(float r) {
   return (uint32_t)r;
 }
 
+// sat_u8_round(roundf(v)), roundf taking halves away from zero: v clamped to
+// [0, 255] (NaN to 0) plus 2^23 is v rounded to the nearest integer, halves
+// to even, in the low bits of the sum; where that took a half down, one more.
+__device__ __forceinline__ uint32_t round_u8(float v) {
+  const float c = fminf(fmaxf(v, 0.0f), 255.0f), y = __fadd_rn(c, 8388608.0f);
+  const float d = __fadd_rn(c, -__fadd_rn(y, -8388608.0f));
+  uint32_t bits;
+#ifdef __CUDA_ARCH__
+  bits = __float_as_uint(y);
+#else
+  std::memcpy(&bits, &y, 4);
+#endif
+  return (bits & 0xFFu) + (d == 0.5f ? 1u : 0u);
+}
+
 // Sample conversions of the f32 path (crates/signinum-j2k-native/src/lib.rs:1772-1840,
 // :2202-2294; crates/signinum-j2k/src/decode.rs:345-356, :517-545).
+// EIGHT: samples of eight bits, rounded and clamped (region request or not);
+// chosen per unit so the hot loop holds no division path.
+template <bool EIGHT>
 __device__ __forceinline__ uint32_t f_to_u8(float v, uint32_t bd, uint32_t region) {
+  if (EIGHT) return round_u8(v);
   const float r = roundf(v);
   if (region) {
     // sample_as_u8: round, clamp to the depth's maximum, rescale to 8 bits.
-    if (bd == 8) return (uint32_t)fminf(fmaxf(r, 0.0f), 255.0f);
     const float maxv = bd >= 16 ? 65535.0f : (float)max((1 << bd) - 1, 1);
     const float c = fminf(fmaxf(r, 0.0f), maxv);
     return sat_u8_round(roundf(__fmul_rn(__fdiv_rn(c, maxv), 255.0f)));
   }
-  // interleave_and_convert: rounded as u8 at 8 bits, else rescaled.
-  if (bd == 8) return sat_u8_round(r);
+  // interleave_and_convert: rescaled.
   return sat_u8_round(roundf(__fmul_rn(__fdiv_rn(v, (float)((1u << bd) - 1)), 255.0f)));
 }
 
@@ -883,17 +888,17 @@ __device__ __forceinline__ uint32_t f_to_u16(float v, uint32_t bd) {
   return (uint32_t)c;
 }
 
-template <int FMT>
+template <int FMT, bool EIGHT>
 __device__ __forceinline__ void put_pixel97(uint32_t* wds, int p, float c0, float c1, float c2, uint32_t bd,
                                             uint32_t reg) {
   constexpr int B = pack_bpp<FMT>();
   const int q = p * B;
   if (FMT == PACK_GRAY8) {
-    put_byte(wds, q, f_to_u8(c0, bd, reg));
+    put_byte(wds, q, f_to_u8<EIGHT>(c0, bd, reg));
   } else if (FMT == PACK_RGB8 || FMT == PACK_RGBA8) {
-    put_byte(wds, q, f_to_u8(c0, bd, reg));
-    put_byte(wds, q + 1, f_to_u8(c1, bd, reg));
-    put_byte(wds, q + 2, f_to_u8(c2, bd, reg));
+    put_byte(wds, q, f_to_u8<EIGHT>(c0, bd, reg));
+    put_byte(wds, q + 1, f_to_u8<EIGHT>(c1, bd, reg));
+    put_byte(wds, q + 2, f_to_u8<EIGHT>(c2, bd, reg));
     if (FMT == PACK_RGBA8) put_byte(wds, q + 3, 255u);
   } else if (FMT == PACK_GRAY16) {
     const uint32_t a = f_to_u16(c0, bd);
@@ -910,13 +915,9 @@ __device__ __forceinline__ void put_pixel97(uint32_t* wds, int p, float c0, floa
   }
 }
 
-// Shared-memory slots of a lane's three-component 9/7 stream: 5 per component
-// (the stream's st(c, 0..4)).
-constexpr int kSlots97 = 5 * 3;
-
-template <int NC, int FMT>
+template <int NC, int FMT, bool EIGHT>
 __device__ __forceinline__ void pack97_unit(const PackJob& job, int x0, int ys, int ye, int lane, uint32_t* rowbuf,
-                                            float4* st, Src97* tab, float IK) {
+                                            Src97* tab, float IK) {
   constexpr int BPP = pack_bpp<FMT>();
   const int w = (int)job.w, h = (int)job.h;
   const int cx0 = (int)job.cx, cy0 = (int)job.cy, cx1 = cx0 + (int)job.cw, cy1 = cy0 + (int)job.ch;
@@ -950,30 +951,30 @@ __device__ __forceinline__ void pack97_unit(const PackJob& job, int x0, int ys, 
         c2 = __fadd_rn(c2, shift);
       }
       c0 = __fadd_rn(c0, shift);
-      put_pixel97<FMT>(wds, p, c0, c1, c2, bd, reg);
+      put_pixel97<FMT, EIGHT>(wds, p, c0, c1, c2, bd, reg);
     }
     // Lane k's words are columns x0 - 4 + 4k ..: the row starts at x0 - 4.
     store_row<BPP>(job.out + (uint64_t)(y - cy0) * job.pitch + (uint64_t)(xs - cx0) * BPP, x0 - 4, xs, nbytes,
                    lane, rowbuf, wds);
   };
   if (job.lifting) {
+    // The components' band descriptors: read from the job once per unit into
+    // the warp's shared table (RGB), or in registers (gray).
+    const bool ll_band = job.ll_band != 0;
+    auto src = [&](int c) {
+      return Src97{job.ll[c], job.hl[c], job.lh[c], job.hh[c], {job.step[c][0], job.step[c][1], job.step[c][2], job.step[c][3]}};
+    };
+    const Src97 one = src(0);
+    bool vec = vec97(one, w, x0 - 4);
     if (NC == 3) {
-      // The components' band descriptors, read from the job once per unit.
-      if (lane < 3)
-        tab[lane] = make_src97(job.ll[lane], job.hl[lane], job.lh[lane], job.hh[lane], job.step[lane],
-                               job.ll_band != 0, w, h, x0 - 4);
+      vec = vec && vec97(src(1), w, x0 - 4) && vec97(src(2), w, x0 - 4);
+      if (lane < 3) tab[lane] = src(lane);
       __syncwarp();
-      stream97<3>([&](int c) -> const Src97& { return tab[c]; }, h, col, ys, ye, kKappa97, IK,
-                  [&](int c, int k) -> float4& { return st[(c * 5 + k) * kLanes + lane]; }, emit);
-      __syncwarp();
-    } else {
-      const Src97 S = make_src97(job.ll[0], job.hl[0], job.lh[0], job.hh[0], job.step[0], job.ll_band != 0, w, h,
-                                 x0 - 4);
-      float4 state[5];
-      const Src97* sp = &S;
-      stream97<1>([sp](int) -> const Src97& { return *sp; }, h, col, ys, ye, kKappa97, IK,
-                  [&](int, int k) -> float4& { return state[k]; }, emit);
     }
+    const Src97* S = NC == 3 ? tab : &one;
+    if (vec) stream97<NC, true>(S, make_cols97<true>(col, w, h, ll_band), ys, ye, kKappa97, IK, emit);
+    else stream97<NC, false>(S, make_cols97<false>(col, w, h, ll_band), ys, ye, kKappa97, IK, emit);
+    if (NC == 3) __syncwarp();  // the table is rewritten by the warp's next unit
   } else {
     // Nothing to lift: the image is the LL band itself (dequantised).
     for (int y = ys; y < ye; ++y) {
@@ -995,15 +996,14 @@ __device__ __forceinline__ void pack97_unit(const PackJob& job, int x0, int ys, 
 
 }  // namespace
 
+// Three CTAs per SM for RGB (142 registers, no spills), five for gray.
 template <int FMT, bool QUEUE>
-__global__ void __launch_bounds__(kWarps97 * 32) pack97_kernel(const PackJob* __restrict__ jobs, uint32_t njobs,
+__global__ void __launch_bounds__(kWarps97 * 32, (FMT == PACK_GRAY8 || FMT == PACK_GRAY16) ? 5 : 3) pack97_kernel(const PackJob* __restrict__ jobs, uint32_t njobs,
                                                                uint32_t nunits, uint32_t* queue) {
   __shared__ __align__(16) uint32_t rowbufs[kWarps97][kRowWords];
-  __shared__ float4 states[kWarps97][kSlots97 * kLanes];
   __shared__ Src97 tabs[kWarps97][3];
   const float IK = __fdiv_rn(1.0f, kKappa97);
   uint32_t* rowbuf = rowbufs[threadIdx.x >> 5];
-  float4* st = states[threadIdx.x >> 5];
   Src97* tab = tabs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   auto one = [&](uint32_t unit) {
@@ -1015,7 +1015,9 @@ __global__ void __launch_bounds__(kWarps97 * 32) pack97_kernel(const PackJob* __
     // RGB formats take RGB tiles, gray formats gray ones (the host maps them
     // so), so the format fixes the component count.
     constexpr int NC = (FMT == PACK_GRAY8 || FMT == PACK_GRAY16) ? 1 : 3;
-    pack97_unit<NC, FMT>(job, x0, ys, ye, lane, rowbuf, st, tab, IK);
+    constexpr bool kU8 = FMT == PACK_GRAY8 || FMT == PACK_RGB8 || FMT == PACK_RGBA8;
+    if (kU8 && job.bit_depth == 8) pack97_unit<NC, FMT, kU8>(job, x0, ys, ye, lane, rowbuf, tab, IK);
+    else pack97_unit<NC, FMT, false>(job, x0, ys, ye, lane, rowbuf, tab, IK);
   };
   if (!QUEUE) {
     const uint32_t unit = blockIdx.x * kWarps97 + (threadIdx.x >> 5);
