@@ -519,13 +519,17 @@ sgn_status build_plan_impl(sgn_ctx* ctx, cudaStream_t s, PinnedBuffer& staging, 
   }
   if (!found_cfg) {
     // Untuned plans: a plan whose last level (or largest IDWT round) has
-    // fewer units than twice the SMs (one tile, a small batch) takes
+    // fewer than 32 units per SM, about two waves of resident warps, takes
     // shorter segments, so that more warps share its rows: down to 4 rows
     // for a 512^2 tile (512 units; 16 rows: 0.165 ms plan latency, 4 rows:
-    // 0.146 ms).
-    const uint32_t sms = (uint32_t)std::max(1, ctx->sm_count);
-    auto shift_for = [&](uint32_t units) {
-      return 4 * units < sms ? -4 : 2 * units < sms ? -3 : units < sms ? -2 : units < 2 * sms ? -1 : 0;
+    // 0.146 ms).  One wave filled in part leaves SMs idle at its end, and a
+    // unit's extra rows (one, or seven at 9/7) cost less: 60 ragged RGBA
+    // tiles (1,600 units) pack 0.11 ms in segments of 64 rows, 0.09 of 16.
+    const uint64_t want = 32ull * (uint64_t)std::max(1, ctx->sm_count);
+    auto shift_for = [&](uint64_t units) {
+      int s = 0;
+      while (s > -4 && (units << -s) < want) --s;
+      return s;
     };
     uint32_t round_units = 0;
     for (const RoundInfo& r : plan->rounds) round_units = std::max(round_units, r.ctas);
