@@ -17,10 +17,36 @@ namespace sgn {
 
 #include "tables/cxtvlc_rows.inc"
 
+// The decoder entries in the form the fused cleanup kernel's chain looks up,
+// with what it needs next already in its place:
+//   CxtVLC: bits 0-4 codeword length, bit 6 u_off, bits 7-9 what the quad adds
+//     to its right neighbour's context, bits 16-31 the packed entry above;
+//   UVLC: bits 0-4 prefix bits, 5-9 prefix and suffix bits, 10-14 the first
+//     quad's suffix bits, 16-20 their mask, 21-25 the second's, 26-28 and
+//     29-31 the two quads' prefix values.
+// A shift count's place in the low five bits of a (shifted) entry needs no
+// mask: shifts take their counts modulo 32.
+struct alignas(16) HtChainTables {
+  uint32_t vlc0[1024], vlc1[1024];
+  uint32_t uvlc0[320], uvlc1[256];
+};
+
+inline uint32_t chain_vlc_entry(uint32_t t, bool initial_row) {
+  const uint32_t right = initial_row ? ((t & 0x10) << 3) | ((t & 0xE0) << 2) : (t & 0xC0) ? 0x100 : 0;
+  return (t & 7) | ((t & 8) << 3) | right | (t << 16);
+}
+
+inline uint32_t chain_uvlc_entry(uint32_t e) {
+  const uint32_t lp = e & 7, len = (e >> 3) & 15, len0 = (e >> 7) & 7, len1 = len - len0;
+  return lp | ((lp + len) << 5) | (len0 << 10) | (((1u << len0) - 1) << 16) | (((1u << len1) - 1) << 21) |
+         (((e >> 10) & 7) << 26) | (((e >> 13) & 7) << 29);
+}
+
 struct HtDecodeTables {
   uint16_t vlc[2][1024];  // [initial row?0:1][(c_q << 7) | next 7 bits]
   uint16_t uvlc0[320];    // initial row: modes 0x00..0x100
   uint16_t uvlc1[256];    // other rows: modes 0x00..0xC0
+  HtChainTables chain;    // the same entries for the fused cleanup kernel
 };
 
 struct HtEncodeEntry {
@@ -86,6 +112,12 @@ inline void build_decode_tables(HtDecodeTables& t) {
     for (uint32_t b = 0; b < 64; ++b) t.uvlc0[m * 64 + b] = uvlc_lookup_entry(m, b, true);
   for (uint32_t m = 0; m < 4; ++m)
     for (uint32_t b = 0; b < 64; ++b) t.uvlc1[m * 64 + b] = uvlc_lookup_entry(m, b, false);
+  for (uint32_t i = 0; i < 1024; ++i) {
+    t.chain.vlc0[i] = chain_vlc_entry(t.vlc[0][i], true);
+    t.chain.vlc1[i] = chain_vlc_entry(t.vlc[1][i], false);
+  }
+  for (uint32_t i = 0; i < 320; ++i) t.chain.uvlc0[i] = chain_uvlc_entry(t.uvlc0[i]);
+  for (uint32_t i = 0; i < 256; ++i) t.chain.uvlc1[i] = chain_uvlc_entry(t.uvlc1[i]);
 }
 
 inline void build_encode_tables(HtEncodeTables& t) {

@@ -28,7 +28,7 @@
 
 namespace sgn {
 
-__device__ HtDecodeTables g_ht_tables;
+__device__ __align__(16) HtDecodeTables g_ht_tables;
 
 namespace {
 
@@ -364,7 +364,6 @@ __device__ __forceinline__ uint32_t left_ctx(uint32_t t) { return ((t & 0xC0u) +
 // (the fused small-plan kernel publishes progress with it).  The row's pairs
 // are staged at stage[pair * stage_stride + stage_slot].
 struct NoRowHook {
-  static constexpr bool kUnroll2 = false;  // the pair loop left to the compiler
   __device__ void operator()(uint32_t) const {}
 };
 template <bool REG, bool OUTLINE, typename RowHook = NoRowHook>
@@ -473,9 +472,7 @@ __device__ bool decode_vlc(const HtJob& job, const uint8_t* src, uint32_t* __res
       pq0 = prev[0] & 0xFFFF;
       pq1 = nq > 1 ? prev[1] & 0xFFFF : 0;
     }
-    // One quad pair of the row (a lambda so that the loop can be unrolled
-    // for one caller only).
-    auto pair_step = [&](uint32_t q) {
+    for (uint32_t q = 0; q < nq; q += 2) {
       uint32_t pq2 = 0, pq3 = 0, a1 = 0;
       if (REG) {
         const uint32_t qc = (uint32_t)Qc;
@@ -531,12 +528,6 @@ __device__ bool decode_vlc(const HtJob& job, const uint8_t* src, uint32_t* __res
         pq0 = pq2;
         pq1 = pq3;
       }
-    };
-    if constexpr (RowHook::kUnroll2) {
-#pragma unroll 2
-      for (uint32_t q = 0; q < nq; q += 2) pair_step(q);
-    } else {
-      for (uint32_t q = 0; q < nq; q += 2) pair_step(q);
     }
     if (REG) S >>= row_align;
     flush();
@@ -832,8 +823,7 @@ struct NoRowWait {
 };
 template <bool NARROW, bool RAW, typename RowWait = NoRowWait>
 __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_words, uint8_t* Ebase, uint32_t cols,
-                            const uint32_t* __restrict__ sym, int32_t* __restrict__ dst,
-                            RowWait row_ready = RowWait()) {
+                            const uint32_t* sym, int32_t* __restrict__ dst, RowWait row_ready = RowWait()) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t w = job.w, h = job.h, stride = job.stride;
   const uint32_t mmsb = job.mmsb, p = 30 - mmsb, mmsbp2 = mmsb + 2, nbp = job.nbp;
@@ -871,8 +861,12 @@ __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_wor
     for (uint32_t c0 = 0; c0 < c0_end; c0 += 32) {
       const uint32_t q = c0 + lane;
       const bool active = q < nq;
-      // Symbols written by the same CTA's chain lane are read past L1.
-      const uint32_t s = active ? (RowWait::kLive ? __ldcg(srow + q) : srow[q]) : 0;
+      // Symbols written by the same CTA's chain lane: in shared memory, or
+      // (wide blocks) read past L1.
+      const uint32_t s = active ? (!RowWait::kLive ? srow[q]
+                                   : NARROW        ? *const_cast<const volatile uint32_t*>(srow + q)
+                                                   : __ldcg(srow + q))
+                                : 0;
       const uint32_t inf = s & 0xFFFF;
       uint32_t U = s >> 16;
       if (!initial) {
@@ -1035,7 +1029,7 @@ namespace {
 // are the warp's shared-memory bit array and exponent rows.
 template <typename RowWait = NoRowWait>
 __device__ void magsgn_block(const HtJob& job, const uint8_t* __restrict__ arena,
-                             const uint32_t* __restrict__ symbols, int32_t* __restrict__ coef,
+                             const uint32_t* symbols, int32_t* __restrict__ coef,
                              uint32_t* __restrict__ tile_status, uint32_t ms_words, uint32_t cols, uint32_t* W,
                              uint8_t* Ebase, RowWait row_ready = RowWait()) {
   const uint32_t lane = threadIdx.x & 31;
@@ -1046,7 +1040,7 @@ __device__ void magsgn_block(const HtJob& job, const uint8_t* __restrict__ arena
       for (uint32_t x = lane; x < w; x += 32) dst[(size_t)y * stride + x] = 0;
     return;
   }
-  const uint32_t* sym = symbols + job.sym;
+  const uint32_t* sym = RowWait::kLive ? symbols : symbols + job.sym;  // (live: the block's own table)
   const uint8_t* src = arena + job.src;
   // The block's cleanup bytes and quad symbols are requested from HBM before
   // the first of them is loaded: the unstuffing steps and the quad rows then
@@ -1203,12 +1197,8 @@ constexpr uint32_t kFusedThreads = 64;
 constexpr uint32_t kRowsFailed = 0xFFFFFFFFu;
 constexpr uint32_t kFusedSpinLimit = 1u << 20;
 
-// The chain lane's row hook: the row's symbols, then its flag.  Its pair
-// loop is unrolled twice (a fused plan runs few chains per SM, each on a
-// warp of its own: 0.146 -> 0.139 ms for a 512^2 tile; the two-pass VLC
-// kernel, 32 chains per warp, is slower unrolled).
+// The chain lane's row hook: the row's symbols, then its flag.
 struct FusedPublish {
-  static constexpr bool kUnroll2 = true;
   volatile uint32_t* progress;
   __device__ void operator()(uint32_t rows) const {
     __threadfence_block();
@@ -1237,30 +1227,248 @@ struct FusedRowWait {
 
 }  // namespace
 
+// The chain of a block at most 64 wide has a warp of its own here, so it is
+// bound by the latency of its dependent steps, not by instructions: it looks
+// up entries that hold what the next step needs in place (HtChainTables),
+// reads its bits from an array that the whole warp unstuffed beforehand, has
+// no branch per quad but the one for MEL runs that end, and leaves its
+// symbols in shared memory: one 512 x 512 RGB tile 0.111 -> 0.092 ms for the
+// kernel (512 pairs of a 64 x 64 block at about 140 ns, 170 before).  The
+// same entries and selects in the 32-blocks-per-warp VLC pass were slower
+// (uneven batch 0.84 -> 0.87 ms, 256 tiles 0.25 -> 0.28): its warps share
+// their issue slots, and the wider tables cost it CTAs.  Making a pair's
+// symbols behind the next pair's first lookup was slower too (0.097 ms).
+namespace {
+
+constexpr uint32_t kChainPairs = 512;  // quad pairs of a block of at most 4096 samples, at most 64 wide
+constexpr uint32_t kChainWords = kChainPairs * 30 / 32 + 8;  // their bits (at most 30 a pair), and words read ahead
+
+// The block's VLC bits (the backward reader's order, VlcT) into B, as many as
+// the chain can take, zeros behind them; by the calling warp.  d: the cleanup
+// segment.  Bit order and overlaps as in unstuff_magsgn; a byte is short here
+// when its low seven bits are all ones and the byte before it is above 0x8F.
+__device__ void unstuff_vlc(const uint8_t* d, uint32_t lcup, uint32_t scup, uint32_t* B) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t i = lane; i < kChainWords; i += 32) B[i] = 0;
+  __syncwarp();
+  const uint32_t b0 = ld8(d + lcup - 2);
+  uint32_t P = 4 - (((b0 >> 4) & 7) == 7 ? 1 : 0);  // bits before the step
+  if (lane == 0) atomicOr(&B[0], b0 >> 4);
+  uint32_t info = (b0 | 0x0F) > 0x8F ? 1u : 0u;  // bit 0: the byte before the step is above 0x8F
+  const uint32_t n = min(scup - 2, 4 * kChainWords);
+  for (uint32_t base = 0; base < n; base += 128) {
+    // The lane's four bytes, the first one lowest.
+    const uint32_t j = base + 4 * lane;
+    const uint8_t* top = d + lcup - 3 - j;  // (formed only where j < n)
+    uint32_t x = 0, bytes = 0;
+    if (j + 4 <= n) {
+      const uintptr_t addr = (uintptr_t)(top - 3);
+      const uint32_t* wp = reinterpret_cast<const uint32_t*>(addr & ~(uintptr_t)3);
+      const uint32_t sh = (uint32_t)(addr & 3);
+      x = __byte_perm(__funnelshift_r(__ldg(wp), sh ? __ldg(wp + 1) : 0u, 8 * sh), 0, 0x0123);
+      bytes = 4;
+    } else if (j < n) {
+      bytes = n - j;
+      x = ld8(top);
+      if (bytes > 1) x |= (uint32_t)ld8(top - 1) << 8;
+      if (bytes > 2) x |= (uint32_t)ld8(top - 2) << 16;
+    }
+    const uint32_t low = x & 0x7F7F7F7Fu;
+    const uint32_t ones = (low + 0x01010101u) & 0x80808080u;       // low seven bits all ones
+    const uint32_t big = (low + 0x70707070u) & x & 0x80808080u;    // above 0x8F
+    uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, big >> 31, 1);
+    if (lane == 0) prev = info;
+    info = __shfl_sync(0xFFFFFFFFu, big >> 31, 31);
+    uint32_t ev = ones & ((big << 8) | (prev << 7));  // short bytes
+    uint32_t at = P + 8 * (j - base), bits = 8 * bytes;
+    if (__any_sync(0xFFFFFFFFu, ev != 0)) {
+      const uint32_t count = (uint32_t)__popc(ev);
+      uint32_t before = 0, total = 0;
+      for (uint32_t t = 1;; ++t) {
+        const uint32_t has = __ballot_sync(0xFFFFFFFFu, count >= t);
+        if (has == 0) break;
+        before += (uint32_t)__popc(has & ((1u << lane) - 1));
+        total += (uint32_t)__popc(has);
+      }
+      at -= before;
+      P -= total;
+      uint64_t v = x;
+      for (uint32_t drops = 0; ev; ev &= ev - 1, ++drops) {
+        const uint32_t end = (uint32_t)__ffs((int)ev) - drops;  // the short byte's end
+        v = (v & ((1ull << end) - 1)) | ((v >> end) << (end - 1));
+      }
+      x = (uint32_t)v;
+    }
+    P += 8 * min(n - base, 128u);
+    const uint32_t wi = at >> 5, sh = at & 31;
+    if (bits && wi + 1 < kChainWords) {
+      atomicOr(&B[wi], x << sh);
+      if (sh) atomicOr(&B[wi + 1], x >> (32 - sh));
+    }
+  }
+  __syncwarp();
+}
+
+// decode_vlc for a lane with a warp of its own: REG blocks, VLC bits from B,
+// symbols into `sym` (shared memory), row_done as there.
+template <bool OUTLINE, typename RowHook>
+__device__ __forceinline__ void chain_vlc(const HtJob& job, const uint8_t* src, uint32_t scup, const HtChainTables& T,
+                                          const uint32_t* B, uint32_t* sym, RowHook row_done) {
+  const uint32_t nq = (job.w + 1u) / 2, qs = sym_row_stride(job.w), h = job.h;
+  MelT<OUTLINE> mel;
+  mel.init(src, job.lcup, scup);
+  int run = mel.get_run();
+  // The bit window: bit `pos` (< 32) of w0 on; w2 is loaded a word ahead.
+  uint32_t w0 = B[0], w1 = B[1], w2 = B[2], pos = 0, next = 3;
+  auto advance = [&](uint32_t n) {
+    pos += n & 31u;
+    const bool over = pos >= 32;
+    w0 = over ? w1 : w0;
+    w1 = over ? w2 : w1;
+    if (over) w2 = B[min(next, kChainWords - 1)];
+    next += over ? 1 : 0;
+    pos &= 31u;
+  };
+  // A quad's entry with its MEL event when its context is zero.
+  auto event = [&](bool zero, uint32_t t) -> uint32_t {
+    if (zero) {
+      run -= 2;
+      if (run != -1) t = 0;
+      if (run < 0) run = mel.get_run();
+    }
+    return t;
+  };
+  uint32_t* row = sym;
+  uint64_t S = 0;
+  const uint32_t row_align = 64 - 4 * ((nq + 1) / 2);
+  // A pair's symbols from its entries and the window behind its codewords:
+  // the packed entries with the u values above them.
+  auto symbols = [&](uint32_t q, uint32_t v, uint32_t t0, uint32_t t1, uint32_t e, uint32_t base) {
+    const uint32_t x = __funnelshift_r(v, 0u, e), y = __funnelshift_r(x, 0u, e >> 10);
+    const uint32_t u0 = base + ((e >> 26) & 7u) + (x & (e >> 16) & 31u), u1 = base + (e >> 29) + (y & (e >> 21) & 31u);
+    *reinterpret_cast<uint2*>(row + q) = make_uint2(__byte_perm(t0, u0, 0x5432), __byte_perm(t1, u1, 0x5432));
+    S = push_nibble(S, pair_nibble(t0 >> 16, t1 >> 16));
+  };
+  {
+    uint32_t c_q = 0;
+    for (uint32_t q = 0; q < nq; q += 2) {
+      uint32_t v = __funnelshift_r(w0, w1, pos);
+      const uint32_t t0 = event(c_q == 0, T.vlc0[c_q + (v & 0x7F)]);
+      c_q = t0 & 0x380u;
+      v = __funnelshift_r(v, 0u, t0);
+      const uint32_t t1 = q + 1 < nq ? event(c_q == 0, T.vlc0[c_q + (v & 0x7F)]) : 0u;
+      c_q = t1 & 0x380u;
+      v = __funnelshift_r(v, 0u, t1);
+      uint32_t mode = (t0 & 0x40u) | ((t1 & 0x40u) << 1);
+      if (mode == 0xC0) {
+        run -= 2;
+        if (run == -1) mode += 0x40;
+        if (run < 0) run = mel.get_run();
+      }
+      const uint32_t e = T.uvlc0[mode + (v & 0x3F)];
+      advance(t0 + t1 + (e >> 5));  // (three counts, at most 30 together, in the low five bits)
+      symbols(q, v, t0, t1, e, 1u);
+    }
+    S >>= row_align;
+    row_done(1u);
+  }
+  for (uint32_t y = 2; y < h; y += 2) {
+    row += qs;
+    uint32_t c_q = 0;
+    uint64_t Qc = (S | (S >> 1)) >> 1;
+    uint32_t up7 = ((uint32_t)S & 1u) << 7;
+    S = 0;
+    for (uint32_t q = 0; q < nq; q += 2) {
+      const uint32_t qc = (uint32_t)Qc;
+      const uint32_t c0 = c_q | up7 | ((qc & 1u) << 9), a1 = (qc & 5u) << 7;
+      up7 = (qc & 4u) << 5;
+      Qc >>= 4;
+      const bool hasB = q + 1 < nq;
+      const uint32_t v = __funnelshift_r(w0, w1, pos);
+      // As if no MEL run ended in this pair: a quad with a zero context takes
+      // no codeword.
+      const bool z0 = c0 == 0;
+      uint32_t t0 = T.vlc1[c0 + (v & 0x7F)];
+      t0 = z0 ? 0u : t0;
+      uint32_t c1 = (t0 & 0x380u) | a1;
+      uint32_t v1 = __funnelshift_r(v, 0u, t0);
+      const bool z1 = c1 == 0;
+      uint32_t t1 = T.vlc1[c1 + (v1 & 0x7F)];
+      t1 = z1 || !hasB ? 0u : t1;
+      const int events = (z0 ? 2 : 0) + (z1 && hasB ? 2 : 0);
+      if (run < events) {
+        // One does: event by event.
+        t0 = event(z0, T.vlc1[c0 + (v & 0x7F)]);
+        c1 = (t0 & 0x380u) | a1;
+        v1 = __funnelshift_r(v, 0u, t0);
+        t1 = hasB ? event(c1 == 0, T.vlc1[c1 + (v1 & 0x7F)]) : 0u;
+      } else {
+        run -= events;
+      }
+      c_q = t1 & 0x380u;
+      const uint32_t v2 = __funnelshift_r(v1, 0u, t1);
+      const uint32_t mode = (t0 & 0x40u) | ((t1 & 0x40u) << 1);
+      const uint32_t e = T.uvlc1[mode + (v2 & 0x3F)];
+      advance(t0 + t1 + (e >> 5));
+      symbols(q, v2, t0, t1, e, 0u);
+    }
+    S >>= row_align;
+    row_done(y / 2 + 1);
+  }
+}
+
+}  // namespace
+
 template <bool OUTLINE>
 __global__ void __launch_bounds__(kFusedThreads) ht_cleanup_fused_kernel(
     const HtJob* __restrict__ jobs, uint32_t njobs, const uint8_t* __restrict__ arena, uint32_t* __restrict__ symbols,
     int32_t* __restrict__ coef, uint32_t* __restrict__ tile_status, uint32_t ms_words, uint32_t max_w) {
-  __shared__ SmemTables T;
-  __shared__ uint2 stage[16];  // the chain lane's pairs of one row of a 64-wide block
+  // The lookup tables: the chain's form for a block at most 64 wide, decode_vlc's
+  // for a wider one.
+  __shared__ __align__(16) uint32_t tables[sizeof(HtChainTables) / 4];
+  __shared__ uint32_t vlc_bits[kChainWords];
+  // The symbol table of a block at most 64 wide (rows padded to even counts);
+  // a wider block's is in global memory.
+  __shared__ __align__(16) uint32_t table[2 * kChainPairs];
   __shared__ uint32_t rows_done;
   extern __shared__ __align__(16) uint8_t smem[];
+  if (blockIdx.x >= njobs) return;
+  const HtJob job = jobs[blockIdx.x];
+  const bool narrow = job.w <= 64;
   {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&g_ht_tables);
-    uint32_t* d = reinterpret_cast<uint32_t*>(&T);
-    for (uint32_t i = threadIdx.x; i < sizeof(SmemTables) / 4; i += blockDim.x) d[i] = src[i];
+    static_assert(sizeof(HtChainTables) % 16 == 0 && sizeof(SmemTables) % 16 == 0 &&
+                  sizeof(SmemTables) <= sizeof(HtChainTables), "copied by 16 bytes");
+    const uint4* from = reinterpret_cast<const uint4*>(narrow ? reinterpret_cast<const uint8_t*>(&g_ht_tables.chain)
+                                                              : reinterpret_cast<const uint8_t*>(&g_ht_tables));
+    const uint32_t n = (narrow ? sizeof(HtChainTables) : sizeof(SmemTables)) / 16;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) reinterpret_cast<uint4*>(tables)[i] = from[i];
   }
   if (threadIdx.x == 0) rows_done = 0;
   __syncthreads();
-  if (blockIdx.x >= njobs) return;
-  const HtJob job = jobs[blockIdx.x];
   volatile uint32_t* progress = &rows_done;
   if (threadIdx.x < 32) {
-    if (threadIdx.x != 0 || job.passes == 0) return;
-    uint32_t* sym = symbols + job.sym;
+    if (job.passes == 0) return;
+    const uint8_t* src = arena + job.src;
     const FusedPublish publish{progress};
-    const bool ok = job.w <= 64 ? decode_vlc<true, OUTLINE>(job, arena + job.src, sym, T, stage, 1, 0, publish)
-                                : decode_vlc<false, OUTLINE>(job, arena + job.src, sym, T, stage, 1, 0, publish);
+    bool ok;
+    if (narrow) {
+      // decode_vlc's checks of the segment.
+      const uint32_t lcup = job.lcup;
+      uint32_t scup = 0;
+      ok = lcup >= 2;
+      if (ok) {
+        scup = ((uint32_t)ld8(src + lcup - 1) << 4) + (ld8(src + lcup - 2) & 0x0F);
+        ok = scup >= 2 && scup <= lcup && scup <= 4079;
+      }
+      if (ok) unstuff_vlc(src, lcup, scup, vlc_bits);
+      if (threadIdx.x != 0) return;
+      if (ok)
+        chain_vlc<OUTLINE>(job, src, scup, *reinterpret_cast<const HtChainTables*>(tables), vlc_bits, table, publish);
+    } else {
+      if (threadIdx.x != 0) return;
+      ok = decode_vlc<false, OUTLINE>(job, src, symbols + job.sym, *reinterpret_cast<const SmemTables*>(tables),
+                                      nullptr, 1, 0, publish);
+    }
     if (!ok) {
       __threadfence_block();
       *progress = kRowsFailed;
@@ -1268,8 +1476,8 @@ __global__ void __launch_bounds__(kFusedThreads) ht_cleanup_fused_kernel(
     return;
   }
   const uint32_t cols = max_w + 4;
-  magsgn_block(job, arena, symbols, coef, tile_status, ms_words, cols, reinterpret_cast<uint32_t*>(smem),
-               smem + (size_t)ms_words * 4, FusedRowWait{progress});
+  magsgn_block(job, arena, narrow ? table : symbols + job.sym, coef, tile_status, ms_words, cols,
+               reinterpret_cast<uint32_t*>(smem), smem + (size_t)ms_words * 4, FusedRowWait{progress});
 }
 
 // ---------------------------------------------------------------------------
