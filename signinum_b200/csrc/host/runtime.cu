@@ -538,13 +538,28 @@ sgn_status build_plan_impl(sgn_ctx* ctx, cudaStream_t s, PinnedBuffer& staging, 
   }
   if (cfg.idwt_seg_shift || cfg.pack_seg_shift) set_segments(plan, idwt, packs, cfg.idwt_seg_shift, cfg.pack_seg_shift);
   plan->nclassic = ncls;
+  size_t cscratch_bytes = 0;
   if (ncls) {
     plan->classic_slot = std::max<uint32_t>(cslot, 1);
     // Blocks in flight per warp: as few as let every block start at once, up
-    // to what a warp's lanes and its pool of column words hold.
+    // to what a warp's lanes and its shared pool of column words hold.  A
+    // plan of more blocks than fit in shared memory at once keeps its words
+    // in global scratch, with more blocks in flight: 80, 128 and 256 tiles of
+    // 512 x 512 RGB (16,800 to 53,760 blocks) 29.2, 39.0 and 72.3 ms in
+    // shared memory, 27.0, 33.4 and 38.0 ms in scratch with 24 lanes (16: 25.9,
+    // 31.7, 41.7; 32: 29.4, 34.4, 38.7); of 32 x 32 blocks 128 tiles 20.9 and
+    // 11.6 ms (32 lanes; 24: 13.1).  Up to there shared memory is the faster
+    // (its words cost no L1 lookup per lane).
     const uint32_t slots = (uint32_t)ctx->sm_count * classic_ctas_per_sm();
-    plan->classic_lanes = std::min((ncls + slots - 1) / slots, classic_max_lanes(plan->classic_slot));
+    const uint32_t max_lanes = classic_max_lanes(plan->classic_slot);
+    plan->classic_lanes = std::min((ncls + slots - 1) / slots, max_lanes);
     plan->classic_ctas = std::min((ncls + plan->classic_lanes - 1) / plan->classic_lanes, slots);
+    if ((uint64_t)slots * max_lanes < ncls) {
+      const uint32_t wide = (uint32_t)ctx->sm_count * classic_scratch_ctas_per_sm();
+      plan->classic_lanes = max_lanes < 32 ? 24 : 32;
+      plan->classic_ctas = std::min((ncls + plan->classic_lanes - 1) / plan->classic_lanes, wide);
+      cscratch_bytes = (size_t)plan->classic_ctas * plan->classic_lanes * plan->classic_slot * sizeof(uint16_t);
+    }
   }
   plan->nqueues = (uint32_t)plan->rounds.size() + 3 + kPackVariants;
 
@@ -561,9 +576,9 @@ sgn_status build_plan_impl(sgn_ctx* ctx, cudaStream_t s, PinnedBuffer& staging, 
   if ((e = staging.ensure(stage_bytes)) != cudaSuccess) return cuda_status(e, "pinned staging");
   {
     // One table arena: the job tables in their staging layout (uploaded by
-    // one copy), then the work-queue counters.
-    const size_t at_q = up16(stage_bytes - at_ht);
-    if ((e = cudaMallocAsync(&plan->d_tables, at_q + up16((size_t)plan->nqueues * 4), s)) != cudaSuccess)
+    // one copy), then the work-queue counters and the classic scratch.
+    const size_t at_q = up16(stage_bytes - at_ht), at_cs = at_q + up16((size_t)plan->nqueues * 4);
+    if ((e = cudaMallocAsync(&plan->d_tables, at_cs + cscratch_bytes, s)) != cudaSuccess)
       return cuda_status(e, "table arena");
     uint8_t* base = static_cast<uint8_t*>(plan->d_tables);
     plan->d_ht = nht ? reinterpret_cast<HtJob*>(base) : nullptr;
@@ -574,6 +589,7 @@ sgn_status build_plan_impl(sgn_ctx* ctx, cudaStream_t s, PinnedBuffer& staging, 
     plan->d_csegs = ncls ? reinterpret_cast<ClassicSeg*>(base + (at_cseg - at_ht)) : nullptr;
     plan->d_gather = gather_total ? base + (at_gather - at_ht) : nullptr;
     plan->d_queue = reinterpret_cast<uint32_t*>(base + at_q);
+    plan->d_cscratch = cscratch_bytes ? reinterpret_cast<uint16_t*>(base + at_cs) : nullptr;
   }
   uint8_t* st = staging.p;
   HtJob* ht = reinterpret_cast<HtJob*>(st + at_ht);
@@ -768,8 +784,9 @@ sgn_status apply_config(sgn_ctx* ctx, sgn_plan* p, const LaunchConfig& in) {
 }
 
 cudaError_t launch_classic_blocks(const sgn_plan* p, cudaStream_t s) {
-  return launch_classic(p->d_classic, p->d_csegs, p->nclassic, p->d_input, p->d_gather, p->d_coef, p->classic_slot,
-                        p->classic_ctas, p->classic_lanes, p->d_queue + p->rounds.size() + 2 + kPackVariants, s);
+  return launch_classic(p->d_classic, p->d_csegs, p->nclassic, p->d_input, p->d_gather, p->d_coef, p->d_cscratch,
+                        p->classic_slot, p->classic_ctas, p->classic_lanes,
+                        p->d_queue + p->rounds.size() + 2 + kPackVariants, s);
 }
 
 cudaError_t launch_round(const sgn_plan* p, size_t k, cudaStream_t s, bool queued, uint32_t ctas, bool lean) {
@@ -809,6 +826,7 @@ void free_plan_buffers(sgn_plan* p, cudaStream_t s) {
   p->d_refine = nullptr;
   p->d_classic = nullptr;
   p->d_csegs = nullptr;
+  p->d_cscratch = nullptr;
   p->d_gather = nullptr;
   p->d_idwt = nullptr;
   p->d_pack = nullptr;

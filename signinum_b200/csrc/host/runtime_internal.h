@@ -182,7 +182,7 @@ struct sgn_plan {
   // Device allocations (stream-ordered pool): the input arena, and two
   // arenas the buffers below are parts of: d_work (coefficients, level
   // planes, quad symbols, tile status) and d_tables (job tables, work-queue
-  // counters).
+  // counters, classic scratch).
   void* d_work = nullptr;
   void* d_tables = nullptr;
   uint8_t* d_input = nullptr;
@@ -195,6 +195,7 @@ struct sgn_plan {
   // Classic (EBCOT) code blocks: jobs, segment table.
   ClassicJob* d_classic = nullptr;
   ClassicSeg* d_csegs = nullptr;
+  uint16_t* d_cscratch = nullptr;  // column words of plans too large for shared memory
   uint8_t* d_gather = nullptr;  // multi-layer classic blocks' data, gathered per block
   uint32_t nclassic = 0, classic_ctas = 0, classic_lanes = 0, classic_slot = 0;
   IdwtJob* d_idwt = nullptr;

@@ -22,8 +22,9 @@
 // under selects, whose independent parts (column step, probability update,
 // renormalisation) overlap.
 //
-// A stripe column's state is one 16-bit word in shared memory (significance,
-// sign, refined and coded flags of its four samples).  A column and its two
+// A stripe column's state is one 16-bit word (significance, sign, refined and
+// coded flags of its four samples) in shared memory, or, for plans of more
+// blocks than that holds at once, in global scratch behind L1.  A column and its two
 // neighbours, each joined with the samples above and below the stripe, hold
 // the whole context window; they sit in registers while the column is coded,
 // and the next column's words are loaded one column ahead.
@@ -36,7 +37,8 @@
 // branches (10.5 M warp instructions per warp), 21.1 ms in this form with 16
 // blocks per warp; one tile (210 blocks, one per warp) 13.7 ms, with all of
 // them in seven warps 18.3 ms.  The same loop with a branch per kind of
-// decision took 27 ms (24 ms for one tile with 16 blocks per warp).
+// decision took 27 ms (24 ms for one tile with 16 blocks per warp).  256
+// tiles (53,760 blocks, words in scratch) 66 -> 38 ms.
 #include <algorithm>
 #include <cstdint>
 
@@ -106,12 +108,13 @@ __device__ __forceinline__ uint8_t sign_byte(uint32_t i) {
 // C.2) for (index, MPS): qe, bits 16..22 the entry after an MPS, 23..29 the
 // entry after an LPS (the MPS switched where the table says so), bit 31 the
 // MPS; entry 2 * index + MPS.
+template <uint32_t POOL>
 struct Tables {
   uint32_t state[94];
   uint8_t zc[3][512];  // zero-coding label by window index (zc_index)
   uint8_t sc[256];     // sign label | xor << 7 by sign index (sign_index)
   uint32_t cx[19][kClassicBlocks];
-  uint16_t cols[kClassicPool];
+  uint16_t cols[POOL];
 };
 
 // The MQ decoder of Annex C (C in the inverted form of the reference).  The
@@ -212,16 +215,18 @@ struct QeTable {
   uint32_t e[47];
 };
 
-// The third-to-last group of parameters: slot_words, the 16-bit words of the
-// plan's largest block (classic_slot_words); lanes, the blocks each warp has
-// in flight (warps x lanes x slot_words at most kClassicPool).
+// slot_words: the 16-bit words of the plan's largest block
+// (classic_slot_words); lanes: the blocks each warp has in flight.  Their
+// column words are in the CTA's shared pool (warps x lanes x slot_words at
+// most kClassicPool), or with SCRATCH in `scratch`, one slot per lane.
+template <bool SCRATCH = false>
 __global__ void __launch_bounds__(128) classic_kernel(const ClassicJob* __restrict__ jobs,
                                                       const ClassicSeg* __restrict__ segs, uint32_t njobs,
                                                       const uint8_t* __restrict__ arena,
                                                       const uint8_t* __restrict__ gather, int32_t* __restrict__ coef,
-                                                      uint16_t* /*scratch*/, uint32_t slot_words, uint32_t* queue,
+                                                      uint16_t* scratch, uint32_t slot_words, uint32_t* queue,
                                                       QeTable qt, uint32_t lanes = 4) {
-  __shared__ Tables t;
+  __shared__ Tables<SCRATCH ? 2 : kClassicPool> t;
   for (uint32_t i = threadIdx.x; i < 94; i += blockDim.x) {
     const uint32_t e = qt.e[i >> 1], mps = i & 1;
     const uint32_t nm = 2 * ((e >> 16) & 0x7Fu) + mps, nl = 2 * ((e >> 23) & 0x7Fu) + (mps ^ (e >> 30));
@@ -242,7 +247,9 @@ __global__ void __launch_bounds__(128) classic_kernel(const ClassicJob* __restri
   const uint32_t lane = threadIdx.x & 31;
   if (lane >= lanes) return;
   const uint32_t id = (threadIdx.x >> 5) * lanes + lane;
-  uint16_t* const slot = t.cols + id * slot_words;
+  uint16_t* const slot =
+      SCRATCH ? scratch + ((size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane) * slot_words
+              : t.cols + id * slot_words;
 
   // The lane's block.
   ClassicJob job;
@@ -461,16 +468,20 @@ __global__ void __launch_bounds__(128) classic_kernel(const ClassicJob* __restri
 }
 
 cudaError_t launch_classic(const ClassicJob* jobs, const ClassicSeg* segs, uint32_t njobs, const uint8_t* arena,
-                           const uint8_t* gather, int32_t* coef, uint32_t slot_words, uint32_t ctas, uint32_t lanes,
-                           uint32_t* queue, cudaStream_t stream) {
+                           const uint8_t* gather, int32_t* coef, uint16_t* scratch, uint32_t slot_words, uint32_t ctas,
+                           uint32_t lanes, uint32_t* queue, cudaStream_t stream) {
   if (njobs == 0) return cudaSuccess;
-  if (!queue || ctas == 0 || lanes == 0 || lanes > kClassicBlocks || lanes * slot_words > kClassicPool)
+  if (!queue || ctas == 0 || lanes == 0 || lanes > kClassicBlocks || (!scratch && lanes * slot_words > kClassicPool))
     return cudaErrorInvalidValue;
   QeTable qt;
   for (int i = 0; i < 47; ++i)
     qt.e[i] = kQe[i] | ((uint32_t)kNmps[i] << 16) | ((uint32_t)kNlps[i] << 23) | ((uint32_t)kSwitch[i] << 30);
-  classic_kernel<<<ctas, kClassicThreads, 0, stream>>>(jobs, segs, njobs, arena, gather, coef, nullptr, slot_words,
-                                                       queue, qt, lanes);
+  if (scratch)
+    classic_kernel<true><<<ctas, kClassicThreads, 0, stream>>>(jobs, segs, njobs, arena, gather, coef, scratch,
+                                                               slot_words, queue, qt, lanes);
+  else
+    classic_kernel<false><<<ctas, kClassicThreads, 0, stream>>>(jobs, segs, njobs, arena, gather, coef, nullptr,
+                                                                slot_words, queue, qt, lanes);
   return cudaGetLastError();
 }
 
@@ -480,7 +491,16 @@ uint32_t classic_max_lanes(uint32_t slot_words) {
 
 uint32_t classic_ctas_per_sm() {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, classic_kernel, kClassicThreads, 0) != cudaSuccess || n < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, classic_kernel<false>, kClassicThreads, 0) != cudaSuccess ||
+      n < 1)
+    n = 1;
+  return (uint32_t)n;
+}
+
+uint32_t classic_scratch_ctas_per_sm() {
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, classic_kernel<true>, kClassicThreads, 0) != cudaSuccess ||
+      n < 1)
     n = 1;
   return (uint32_t)n;
 }

@@ -76,12 +76,14 @@ cudaError_t idwt_pack_occupancy(uint32_t fmt, int* idwt_ctas_per_sm, int* pack_c
 // Classic (EBCOT Tier-1) code blocks: a persistent grid of `ctas` CTAs of one
 // warp, whose first `lanes` lanes (at most classic_max_lanes) each take blocks
 // from the zeroed counter `queue`; slot_words: classic_slot_words of the
-// largest block.
+// largest block.  scratch: null, the blocks' column words in shared memory;
+// otherwise in ctas x lanes slots of slot_words there (lanes up to 32).
 cudaError_t launch_classic(const ClassicJob* jobs, const ClassicSeg* segs, uint32_t njobs, const uint8_t* arena,
-                           const uint8_t* gather, int32_t* coef, uint32_t slot_words, uint32_t ctas, uint32_t lanes,
-                           uint32_t* queue, cudaStream_t stream);
-uint32_t classic_max_lanes(uint32_t slot_words);
-uint32_t classic_ctas_per_sm();  // resident CTAs per SM of the classic kernel
+                           const uint8_t* gather, int32_t* coef, uint16_t* scratch, uint32_t slot_words, uint32_t ctas,
+                           uint32_t lanes, uint32_t* queue, cudaStream_t stream);
+uint32_t classic_max_lanes(uint32_t slot_words);  // with the column words in shared memory
+uint32_t classic_ctas_per_sm();          // resident CTAs per SM of that form of the kernel
+uint32_t classic_scratch_ctas_per_sm();  // and of the one with the words in scratch
 // Irreversible (9/7) forms of the two launches above, same arguments; the
 // pack units of launch_pack97 run four warps per CTA.
 cudaError_t launch_idwt97_level(const IdwtJob* jobs, uint32_t njobs, uint32_t nunits, cudaStream_t stream,

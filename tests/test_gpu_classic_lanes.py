@@ -23,3 +23,18 @@ def test_many_blocks_lossless(w, h, cb, cb_h, style):
     cs = encode.encode_classic(px, w, h, 3, 8, style=style, levels=3, cb_exp=cb, cb_exp_h=cb_h)
     s = Codec.decode_tile_to_device(cs, PixelFormat.Rgb8, BackendRequest.Cuda)
     assert np.array_equal(np.frombuffer(s.to_bytes(), np.uint8), px)
+
+
+def test_large_and_many_small_blocks_in_one_plan():
+    """A 64 x 64 block sets the slot size of a plan whose 29,000 small blocks
+    then exceed what shared memory holds at once."""
+    from signinum_b200 import encode
+    from signinum_b200.j2k_cuda import BackendRequest, Codec, PixelFormat
+
+    tiles, pixels = [], []
+    for w, h, cb, levels in ((64, 64, 4, 0), (509, 303, 0, 2), (130, 70, 4, 1)):
+        px = encode.he_rgb8(w + h, w, h, 5.0)
+        tiles.append(encode.encode_classic(px, w, h, 3, 8, levels=levels, cb_exp=cb))
+        pixels.append(px)
+    for s, px in zip(Codec.decode_tiles_to_device(tiles, PixelFormat.Rgb8, BackendRequest.Cuda), pixels):
+        assert np.array_equal(np.frombuffer(s.to_bytes(), np.uint8), px)
