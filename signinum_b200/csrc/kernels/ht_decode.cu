@@ -1255,7 +1255,9 @@ __device__ void unstuff_vlc(const uint8_t* d, uint32_t lcup, uint32_t scup, uint
   uint32_t P = 4 - (((b0 >> 4) & 7) == 7 ? 1 : 0);  // bits before the step
   if (lane == 0) atomicOr(&B[0], b0 >> 4);
   uint32_t info = (b0 | 0x0F) > 0x8F ? 1u : 0u;  // bit 0: the byte before the step is above 0x8F
-  const uint32_t n = min(scup - 2, 4 * kChainWords);
+  // As many bytes as hold the chain's bits at seven bits a byte.
+  const uint32_t n = min(scup - 2, 5 * kChainWords);
+  static_assert(7 * 5 * kChainWords >= 32 * (kChainWords - 4), "seven bits a byte cover what the chain takes");
   for (uint32_t base = 0; base < n; base += 128) {
     // The lane's four bytes, the first one lowest.
     const uint32_t j = base + 4 * lane;
