@@ -996,7 +996,7 @@ __device__ __forceinline__ void pack97_unit(const PackJob& job, int x0, int ys, 
 
 }  // namespace
 
-// Three CTAs per SM for RGB (142 registers, no spills), five for gray.
+// Three CTAs per SM for RGB (152 registers, no spills), five for gray.
 template <int FMT, bool QUEUE>
 __global__ void __launch_bounds__(kWarps97 * 32, (FMT == PACK_GRAY8 || FMT == PACK_GRAY16) ? 5 : 3) pack97_kernel(const PackJob* __restrict__ jobs, uint32_t njobs,
                                                                uint32_t nunits, uint32_t* queue) {
