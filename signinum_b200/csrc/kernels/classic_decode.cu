@@ -148,10 +148,13 @@ struct MqDec {
     a = 0x8000;
   }
   // One decision with a context whose state is e; an e of 0 changes nothing
-  // and gives 0.  *cx receives the context's next state.
+  // and gives 0.  *cx receives the context's next state.  (In a valid stream
+  // C stays below A.  A byte 0x80 .. 0x8F after 0xFF can take bytein below
+  // zero, as it does in the reference, so an e of 0 is told apart by its q and
+  // not by C: A is then never 0, and the renormalisation shifts by at most 15.)
   __device__ __forceinline__ uint32_t decode(uint32_t e, uint32_t* cx, const uint32_t* state) {
     const uint32_t q = e & 0xFFFFu, rest = a - q;
-    const bool low = (c >> 16) >= rest;   // the LPS sub-interval
+    const bool low = q != 0 && (c >> 16) >= rest;  // the LPS sub-interval
     const bool lps = low != (rest < q);   // with the conditional exchange
     c -= low ? rest << 16 : 0u;
     a = low ? q : rest;

@@ -6,11 +6,13 @@
 // offsets and the refinement list, one IDWT job per component and level,
 // one pack job).  The coefficients after the HT kernels are compared with
 // the oracle's block decoder, the pixels with the oracle's decode.  Usage:
-// emu <pixel formats, e.g. 134> <codestream>...; prints one line per codestream and
-// exits non-zero on any difference.
+// emu <pixel formats, e.g. 134> [-d SEED] <codestream>...; prints one line per codestream and
+// exits non-zero on any difference.  -d: the classic code blocks' data is damaged
+// first (damage_segments).
 #include <fstream>
 #include <iterator>
 #include <memory>
+#include <random>
 #include <thread>
 #include <vector>
 #include "cuda_shim.h"
@@ -338,15 +340,52 @@ int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts) {
   return (nd_total || cdiff) ? 1 : 0;
 }
 
+// Writes byte pairs FF 80 .. FF 8F, after which the MQ decoder takes more than
+// its C register may hold, into every codeword segment of a classic
+// codestream, seeded: at its start, behind a run of FF 7F pairs (which leaves
+// C at zero, so that the pair underflows it in mid-stream), or at random
+// places.  The packet headers stay as they are.
+static void damage_segments(std::vector<uint8_t>& d, uint32_t seed) {
+  sgn::TileLayout T;
+  sgn::parse_tile(d.data(), d.size(), nullptr, T);
+  std::mt19937 rng(seed);
+  for (const sgn::CodeBlock& cb : T.blocks) {
+    if (!cb.passes) continue;
+    size_t at = cb.cleanup_off;
+    for (uint32_t k = 0; k < cb.nseg; ++k) {
+      const size_t len = T.segments[cb.seg_begin + k].len;
+      uint8_t* s = d.data() + at;
+      at += len;
+      if (len < 2) continue;
+      const uint32_t kind = rng() % 4;
+      if (kind == 3) {
+        for (uint32_t n = 1 + rng() % 4; n; --n) {
+          const size_t o = rng() % (len - 1);
+          s[o] = 0xFF;
+          s[o + 1] = (uint8_t)(0x80 + rng() % 16);
+        }
+        continue;
+      }
+      size_t o = 0;
+      for (uint32_t n = kind == 2 ? 1 + rng() % 6 : 0; n && o + 4 <= len; --n, o += 2) s[o] = 0xFF, s[o + 1] = 0x7F;
+      s[o] = 0xFF;
+      s[o + 1] = (uint8_t)(0x80 + rng() % 16);
+    }
+  }
+}
+
 int main(int argc, char** argv) {
   sgn::emu_tables();
   std::vector<int> fmts;
   for (const char* c = argv[1]; *c; ++c)
     if (*c >= '0' && *c <= '4') fmts.push_back(*c - '0');
-  int fails = 0;
-  for (int i = 2; i < argc; ++i) {
+  int fails = 0, first = 2;
+  const bool damaged = argc > 3 && !std::strcmp(argv[2], "-d");
+  if (damaged) first = 4;
+  for (int i = first; i < argc; ++i) {
     std::ifstream f(argv[i], std::ios::binary);
     std::vector<uint8_t> d((std::istreambuf_iterator<char>(f)), {});
+    if (damaged) damage_segments(d, (uint32_t)std::atoi(argv[3]) + (uint32_t)i);
     fails += run(d, fmts) != 0;
   }
   printf("fails %d\n", fails);

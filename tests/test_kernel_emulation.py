@@ -39,13 +39,13 @@ def emu(tmp_path_factory):
     return out
 
 
-def run(emu, fmts, codestreams):
+def run(emu, fmts, codestreams, options=(), timeout=600):
     paths = []
     for k, cs in enumerate(codestreams):
         p = emu / f"case_{fmts}_{k}.j2k"
         p.write_bytes(cs)
         paths.append(str(p))
-    r = subprocess.run([str(emu / "emu"), fmts] + paths, capture_output=True, text=True, timeout=600)
+    r = subprocess.run([str(emu / "emu"), fmts, *options] + paths, capture_output=True, text=True, timeout=timeout)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
     assert r.stdout.strip().endswith("fails 0")
 
@@ -110,3 +110,24 @@ def test_interior_strips_through_emulated_kernels(emu):
                                                       cb_exp=4, cb_exp_h=3))
     run(emu, "03", by_comps[1])
     run(emu, "124", by_comps[3])
+
+
+@pytest.mark.parametrize("style", [0x00, 0x01, 0x02, 0x04, 0x05, 0x08, 0x2F])
+def test_damaged_classic_segments_through_emulated_kernels(emu, style):
+    """FF 80 .. FF 8F at the start of codeword segments and inside them: the
+    MQ decoder's C register underflows there, and an iteration of the kernel
+    that codes no sample must leave the decoder as it is all the same.
+    Coefficients and pixels equal the oracle's; the time limit fails a decoder
+    that such a pair sends into a loop."""
+    from signinum_b200 import encode
+    from tests.helpers import random_tile
+
+    rng = np.random.default_rng(4600 + style)
+    streams = []
+    for w, h, cb, cb_h, levels in [(24, 24, 4, 4, 0), (33, 18, 3, 1, 0), (40, 29, 2, 2, 1), (9, 70, 0, 4, 0),
+                                   (130, 7, 6, 2, 0), (64, 64, 4, 4, 0)]:
+        px = random_tile(rng, w, h, 1, 8, int(rng.integers(0, 2)))
+        streams.append(encode.encode_classic(px.reshape(-1), w, h, 1, 8, style=style, levels=levels, cb_exp=cb,
+                                             cb_exp_h=cb_h))
+    for seed in (1, 100):
+        run(emu, "0", streams, ["-d", str(seed)], timeout=60)
