@@ -51,8 +51,8 @@ namespace {
 
 using namespace ebcot;
 
-// One warp per CTA in the launches below; at most 32 blocks in flight per
-// CTA, whose column words share one pool (16 blocks of 64 x 64).
+// One warp per CTA; at most 32 blocks in flight per CTA, whose column words
+// share one pool (16 blocks of 64 x 64).
 constexpr uint32_t kClassicThreads = 32, kClassicBlocks = 32;
 constexpr uint32_t kClassicPool = 16 * classic_slot_words(64, 64);
 
@@ -219,16 +219,14 @@ struct QeTable {
 };
 
 // slot_words: the 16-bit words of the plan's largest block
-// (classic_slot_words); lanes: the blocks each warp has in flight.  Their
-// column words are in the CTA's shared pool (warps x lanes x slot_words at
-// most kClassicPool), or with SCRATCH in `scratch`, one slot per lane.
-template <bool SCRATCH = false>
-__global__ void __launch_bounds__(128) classic_kernel(const ClassicJob* __restrict__ jobs,
-                                                      const ClassicSeg* __restrict__ segs, uint32_t njobs,
-                                                      const uint8_t* __restrict__ arena,
-                                                      const uint8_t* __restrict__ gather, int32_t* __restrict__ coef,
-                                                      uint16_t* scratch, uint32_t slot_words, uint32_t* queue,
-                                                      QeTable qt, uint32_t lanes = 4) {
+// (classic_slot_words); lanes: the blocks the CTA's warp has in flight.  Their
+// column words are in the CTA's shared pool (lanes x slot_words at most
+// kClassicPool), or with SCRATCH in `scratch`, one slot per lane.
+template <bool SCRATCH>
+__global__ void __launch_bounds__(kClassicThreads) classic_kernel(
+    const ClassicJob* __restrict__ jobs, const ClassicSeg* __restrict__ segs, uint32_t njobs,
+    const uint8_t* __restrict__ arena, const uint8_t* __restrict__ gather, int32_t* __restrict__ coef,
+    uint16_t* scratch, uint32_t slot_words, uint32_t* queue, QeTable qt, uint32_t lanes) {
   __shared__ Tables<SCRATCH ? 2 : kClassicPool> t;
   for (uint32_t i = threadIdx.x; i < 94; i += blockDim.x) {
     const uint32_t e = qt.e[i >> 1], mps = i & 1;
@@ -247,12 +245,10 @@ __global__ void __launch_bounds__(128) classic_kernel(const ClassicJob* __restri
     t.sc[i] = (uint8_t)(label | (xr << 7));
   }
   __syncthreads();
-  const uint32_t lane = threadIdx.x & 31;
-  if (lane >= lanes) return;
-  const uint32_t id = (threadIdx.x >> 5) * lanes + lane;
+  const uint32_t id = threadIdx.x;
+  if (id >= lanes) return;
   uint16_t* const slot =
-      SCRATCH ? scratch + ((size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane) * slot_words
-              : t.cols + id * slot_words;
+      SCRATCH ? scratch + ((size_t)blockIdx.x * lanes + id) * slot_words : t.cols + id * slot_words;
 
   // The lane's block.
   ClassicJob job;

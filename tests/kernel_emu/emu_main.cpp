@@ -37,7 +37,8 @@ void emu_idwt(bool, const IdwtJob*, uint32_t, uint32_t);
 void emu_pack(bool, int, const PackJob*, uint32_t, uint32_t);
 int emu_pack_warps(bool);
 void emu_classic(const ClassicJob*, const ClassicSeg*, uint32_t, const uint8_t*, const uint8_t*, int32_t*, uint16_t*,
-                 uint32_t, uint32_t*);
+                 uint32_t, uint32_t*, uint32_t);
+uint32_t emu_classic_max_lanes(uint32_t);
 size_t ht_magsgn_smem_bytes(uint32_t ms_words, uint32_t max_w, uint32_t warps);
 }
 extern "C" int oracle_decode(const uint8_t*, size_t, int, int, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t,
@@ -133,14 +134,31 @@ int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts) {
         for (uint32_t x = 0; x < cb.w; ++x) ref[j.dst + (size_t)y * b.w + x] = blk[(size_t)y * cb.w + x];
     }
     n = (uint32_t)cj.size();
-    const uint32_t ctas = std::min<uint32_t>((n + 127) / 128, 2);
-    std::vector<uint16_t> scratch((size_t)std::max<uint32_t>(ctas, 1) * 128 * slot, 0xABCD);
-    std::vector<uint32_t> queue(1, 0);
-    if (n)
-      launch(ctas, 128, [&] {
-        emu_classic(cj.data(), cs.data(), n, arena.data(), gather.data(), coef.data(), scratch.data(), slot,
-                    queue.data());
+    // The launch's forms: CTAs of one warp with 1, a few or as many blocks in
+    // flight as the shared pool holds, and with the column words in scratch (24
+    // and 32 lanes).  CTAs run one after the other here, so each takes a share
+    // of the blocks through a counter of its own.
+    const uint32_t most = emu_classic_max_lanes(slot);
+    const struct { bool in_scratch; uint32_t lanes; } forms[] = {{false, 1}, {false, std::min(5u, most)}, {false, most},
+                                                                 {true, 24}, {true, 32}};
+    std::vector<int32_t> first;
+    for (const auto& f : forms) {
+      std::fill(coef.begin(), coef.end(), 0x7F7F7F7F);
+      const uint32_t ctas = std::max(1u, std::min((n + f.lanes - 1) / f.lanes, 3u));
+      std::vector<uint16_t> scratch(f.in_scratch ? (size_t)ctas * f.lanes * slot : 0, 0xABCD);
+      std::vector<uint32_t> queue;
+      for (uint32_t b = 0; b < ctas; ++b) queue.push_back((uint32_t)((uint64_t)n * b / ctas));
+      launch(n ? ctas : 0, 32, [&] {
+        const uint32_t b = blockIdx.x;
+        emu_classic(cj.data(), cs.data(), (uint32_t)((uint64_t)n * (b + 1) / ctas), arena.data(), gather.data(),
+                    coef.data(), f.in_scratch ? scratch.data() : nullptr, slot, &queue[b], f.lanes);
       });
+      if (first.empty()) first = coef;
+      else if (coef != first) {
+        printf("classic kernel forms disagree (%u lanes%s)\n", f.lanes, f.in_scratch ? ", scratch" : "");
+        return 1;
+      }
+    }
   } else {
   // HT jobs (runtime passes A/B for one tile).
   std::vector<HtJob> jobs;
@@ -348,6 +366,7 @@ int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts) {
 static void damage_segments(std::vector<uint8_t>& d, uint32_t seed) {
   sgn::TileLayout T;
   sgn::parse_tile(d.data(), d.size(), nullptr, T);
+  if (!T.classic || T.gathered) std::abort();  // the offsets below are the codestream's
   std::mt19937 rng(seed);
   for (const sgn::CodeBlock& cb : T.blocks) {
     if (!cb.passes) continue;

@@ -33,13 +33,16 @@ void emu_fused(const HtJob* jobs, uint32_t n, const uint8_t* arena, uint32_t* sy
 
 CLASSIC_WRAPPERS = """
 namespace sgn {
+uint32_t emu_classic_max_lanes(uint32_t slot) { return classic_max_lanes(slot); }
 void emu_classic(const ClassicJob* jobs, const ClassicSeg* segs, uint32_t n, const uint8_t* arena,
-                 const uint8_t* gather, int32_t* coef, uint16_t* scratch, uint32_t slot, uint32_t* queue) {
+                 const uint8_t* gather, int32_t* coef, uint16_t* scratch, uint32_t slot, uint32_t* queue,
+                 uint32_t lanes) {
   QeTable qt;
   for (int i = 0; i < 47; ++i)
     qt.e[i] = ebcot::kQe[i] | ((uint32_t)ebcot::kNmps[i] << 16) | ((uint32_t)ebcot::kNlps[i] << 23) |
               ((uint32_t)ebcot::kSwitch[i] << 30);
-  classic_kernel(jobs, segs, n, arena, gather, coef, scratch, slot, queue, qt);
+  if (scratch) classic_kernel<true>(jobs, segs, n, arena, gather, coef, scratch, slot, queue, qt, lanes);
+  else classic_kernel<false>(jobs, segs, n, arena, gather, coef, nullptr, slot, queue, qt, lanes);
 }
 }  // namespace sgn
 """
@@ -107,7 +110,6 @@ def main(out_dir):
     src = src.replace('#include "../device_plan.h"', inc("device_plan.h")).replace('#include "../ebcot.h"', inc("ebcot.h"))
     src = src.replace('#include "kernels.h"', '#include "cuda_shim.h"')
     src = strip_functions(src, r"launch_\w+")
-    src = re.sub(r"^uint32_t classic_threads_per_cta\(\) \{[^}]*\}", "", src, flags=re.M)
     src = src[:src.index("uint32_t classic_ctas_per_sm()")] + "}  // namespace sgn\n"
     (out / "classic_emu.cpp").write_text(src + CLASSIC_WRAPPERS)
 

@@ -2,7 +2,12 @@
 every HT, classic (EBCOT), IDWT and pack kernel on the golden fixtures and
 on seeded random reversible, irreversible and classic codestreams, built with AddressSanitizer, and
 compared with the oracle (coefficients per code block, then pixels, exact).
-Out-of-bounds accesses and parity breaks show up here without a GPU."""
+The classic kernel runs as it is launched: CTAs of one warp with 1, 5 or as
+many blocks in flight as its shared pool holds, and with 24 and 32 blocks
+whose column words are in scratch.  Out-of-bounds accesses and parity breaks
+show up here without a GPU.  Three helpers that are inline PTX on the device
+(the warp scan, the predicated load, the saturating pack) run their C++ forms
+here; the PTX forms are compared by the GPU tests alone."""
 import json
 import pathlib
 import shutil
