@@ -21,6 +21,7 @@
 // blocks that carry them.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "../device_plan.h"
 #include "../ht_tables.h"
@@ -719,10 +720,12 @@ struct QuadBits {
 // U is the quad's u_q (plus the exponent bound kappa after the first row);
 // U > mmsb + 2 marks an invalid stream, which the caller flags and whose
 // block comes out as zeros, so clamping U to 31 here (the bytes then cannot
-// carry) changes no valid result.
-__device__ __forceinline__ QuadBits quad_bits(uint32_t inf, uint32_t U) {
+// carry) changes no valid result.  right: the quad's right column lies in the
+// block; where it does not (the last quad of an odd width) a damaged stream
+// can make its samples significant, and they take no bits of the stream.
+__device__ __forceinline__ QuadBits quad_bits(uint32_t inf, uint32_t U, bool right) {
   const uint32_t sig = spread4((inf >> 4) & 0xFu), k = spread4(inf >> 12);
-  const uint32_t m = (min(U, 31u) * 0x01010101u - k) & (sig * 0xFFu);
+  const uint32_t m = (min(U, 31u) * 0x01010101u - k) & (sig * 0xFFu) & (right ? ~0u : 0xFFFFu);
   return QuadBits{m, m * 0x01010101u};
 }
 
@@ -814,14 +817,16 @@ __device__ __forceinline__ void quad_samples(const uint32_t* W, uint32_t ms_word
 // wide, one quad per lane per row) they stay in registers and come from the
 // neighbouring lanes by shuffles, otherwise they are kept per column in
 // shared memory (Ebase, two rows of `cols` bytes).  Returns true (on every
-// lane) when the stream is invalid.
+// lane) when the stream is invalid.  ODD: the width may be odd (quad_bits); the
+// usual even widths keep a loop without that test, which took 1 % of the
+// uneven batch's pass (2.175 -> 2.195 ms).
 // Rows are taken as they are: the two-pass form decodes symbols a kernel
 // earlier.
 struct NoRowWait {
   static constexpr bool kLive = false;
   __device__ bool operator()(uint32_t) const { return true; }
 };
-template <bool NARROW, bool RAW, typename RowWait = NoRowWait>
+template <bool NARROW, bool RAW, bool ODD, typename RowWait = NoRowWait>
 __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_words, uint8_t* Ebase, uint32_t cols,
                             const uint32_t* sym, int32_t* __restrict__ dst, RowWait row_ready = RowWait()) {
   const uint32_t lane = threadIdx.x & 31;
@@ -893,7 +898,7 @@ __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_wor
       }
       // (A lane without a quad holds U of 0 or 1 and no significant sample.)
       bad |= U > mmsbp2;
-      const QuadBits qb = quad_bits(inf, U);
+      const QuadBits qb = quad_bits(inf, U, !ODD || 2 * q + 1 < w);
       const uint32_t tot = qb.incl >> 24;
       const uint32_t inc = inclusive_scan<32>(tot);
       const uint32_t off = rowbase + inc - tot;
@@ -952,9 +957,10 @@ __device__ bool magsgn_rows(const HtJob& job, const uint32_t* W, uint32_t ms_wor
 // trip counts (a half past its own work idles), so no warp-synchronous
 // operation sits in a branch that one half skips.
 
-// magsgn_rows<true, false> for the calling half-warp's block (live) over
+// magsgn_rows<true, false, ODD> for the calling half-warp's block (live) over
 // hmax rows, the taller of the two blocks' heights.  Returns true on the
 // half's lanes when its stream is invalid.
+template <bool ODD>
 __device__ bool magsgn_rows_half(const HtJob& job, bool live, const uint32_t* W, uint32_t ms_words, uint32_t hmax,
                                  const uint32_t* __restrict__ sym, int32_t* __restrict__ dst) {
   const uint32_t lane = threadIdx.x & 31, gl = lane & 15, gsh = lane & 16;
@@ -989,7 +995,7 @@ __device__ bool magsgn_rows_half(const HtJob& job, bool live, const uint32_t* W,
       U += gamma != 0 ? max(e, 1u) : 1u;
     }
     bad |= U > mmsbp2;
-    const QuadBits qb = quad_bits(inf, U);
+    const QuadBits qb = quad_bits(inf, U, !ODD || has_right);
     const uint32_t tot = qb.incl >> 24;
     const uint32_t inc = inclusive_scan<16>(tot);
     const uint32_t off = rowbase + inc - tot;
@@ -1072,11 +1078,18 @@ __device__ void magsgn_block(const HtJob& job, const uint8_t* __restrict__ arena
     unstuff_magsgn<32>(src, ms_len, W, words);
     // Blocks with refinement passes keep the sign-magnitude words for them.
     const bool raw = job.passes > 1;
-    const bool bad =
-        job.w <= 64 ? (raw ? magsgn_rows<true, true>(job, W, words, Ebase, cols, sym, dst, row_ready)
-                           : magsgn_rows<true, false>(job, W, words, Ebase, cols, sym, dst, row_ready))
-                    : (raw ? magsgn_rows<false, true>(job, W, words, Ebase, cols, sym, dst, row_ready)
-                           : magsgn_rows<false, false>(job, W, words, Ebase, cols, sym, dst, row_ready));
+    auto rows = [&](auto narrow, auto raw_words, auto odd) {
+      return magsgn_rows<decltype(narrow)::value, decltype(raw_words)::value, decltype(odd)::value>(
+          job, W, words, Ebase, cols, sym, dst, row_ready);
+    };
+    using T = std::true_type;
+    using F = std::false_type;
+    // One loop for every width where the block is rare or waits for its chain.
+    const bool narrow = job.w <= 64;
+    bool bad;
+    if (raw) bad = narrow ? rows(T{}, T{}, T{}) : rows(F{}, T{}, T{});
+    else if (RowWait::kLive || (job.w & 1)) bad = narrow ? rows(T{}, F{}, T{}) : rows(F{}, F{}, T{});
+    else if constexpr (!RowWait::kLive) bad = narrow ? rows(T{}, F{}, F{}) : rows(F{}, F{}, F{});
     ok = !bad;
   }
   if (!ok) {
@@ -1122,7 +1135,9 @@ __device__ void magsgn_pair(const HtJob* __restrict__ jobs, uint32_t a, uint32_t
   unstuff_magsgn<16>(src, ms_len, Wg, words);
   const uint32_t hh = ok ? job.h : 0;
   const uint32_t hmax = max(hh, __shfl_xor_sync(0xFFFFFFFFu, hh, 16));
-  const bool bad = magsgn_rows_half(job, ok, Wg, words, hmax, sym, dst);
+  const bool odd = __any_sync(0xFFFFFFFFu, job.w & 1);
+  const bool bad = odd ? magsgn_rows_half<true>(job, ok, Wg, words, hmax, sym, dst)
+                       : magsgn_rows_half<false>(job, ok, Wg, words, hmax, sym, dst);
   if (present && (!ok || bad)) {
     // No coded passes: zeros; an invalid stream: zeros and the tile's status.
     for (uint32_t y = 0; y < job.h; ++y)

@@ -7,8 +7,9 @@
 // one pack job).  The coefficients after the HT kernels are compared with
 // the oracle's block decoder, the pixels with the oracle's decode.  Usage:
 // emu <pixel formats, e.g. 134> [-d SEED] <codestream>...; prints one line per codestream and
-// exits non-zero on any difference.  -d: the classic code blocks' data is damaged
-// first (damage_segments).
+// exits non-zero on any difference.  -d: the code blocks' data is damaged first
+// (damage_segments, damage_cleanup); where the oracle rejects the damaged
+// codestream, the kernels must have set its status.
 #include <fstream>
 #include <iterator>
 #include <memory>
@@ -75,7 +76,7 @@ static int32_t to_i32(uint32_t v, uint32_t nbp) {
 }
 static int bpp_of(int f) { return f == 0 ? 1 : f == 1 ? 3 : f == 2 ? 4 : f == 3 ? 2 : 6; }
 
-int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts) {
+int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts, bool damaged) {
   using namespace sgn;
   TileLayout T;
   try {
@@ -345,7 +346,10 @@ int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts) {
     std::vector<uint8_t> want((size_t)W * H * bpp + 16);
     uint32_t ow, oh;
     int rc = oracle_decode(d.data(), d.size(), fmt, 0, 0, 0, 0, 0, 1, want.data(), want.size(), &ow, &oh);
-    if (rc) { printf("oracle error %d\n", rc); return 2; }
+    if (rc) {
+      printf("oracle error %d, status %u\n", rc, status[0]);
+      return damaged && status[0] ? 0 : 2;
+    }
     size_t nd = 0, first = SIZE_MAX;
     for (size_t i = 0; i < (size_t)W * H * bpp; ++i)
       if (out[i] != want[i]) { ++nd; if (first == SIZE_MAX) first = i; }
@@ -355,7 +359,7 @@ int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts) {
     printf("\n");
     nd_total += nd;
   }
-  return (nd_total || cdiff) ? 1 : 0;
+  return (nd_total || cdiff || status[0]) ? 1 : 0;
 }
 
 // Writes byte pairs FF 80 .. FF 8F, after which the MQ decoder takes more than
@@ -366,7 +370,7 @@ int run(const std::vector<uint8_t>& d, const std::vector<int>& fmts) {
 static void damage_segments(std::vector<uint8_t>& d, uint32_t seed) {
   sgn::TileLayout T;
   sgn::parse_tile(d.data(), d.size(), nullptr, T);
-  if (!T.classic || T.gathered) std::abort();  // the offsets below are the codestream's
+  if (T.gathered) std::abort();  // the offsets below are the codestream's
   std::mt19937 rng(seed);
   for (const sgn::CodeBlock& cb : T.blocks) {
     if (!cb.passes) continue;
@@ -393,6 +397,23 @@ static void damage_segments(std::vector<uint8_t>& d, uint32_t seed) {
   }
 }
 
+// Changes a few bytes of every HT cleanup segment, seeded: near its end, where
+// the MEL and VLC bits are, or anywhere.
+static void damage_cleanup(std::vector<uint8_t>& d, uint32_t seed) {
+  sgn::TileLayout T;
+  sgn::parse_tile(d.data(), d.size(), nullptr, T);
+  std::mt19937 rng(seed);
+  for (const sgn::CodeBlock& cb : T.blocks) {
+    if (!cb.passes || cb.lcup < 6) continue;
+    uint8_t* s = d.data() + cb.cleanup_off;
+    for (uint32_t n = 1 + rng() % 3; n; --n) {
+      // (The last two bytes hold the segment's own lengths.)
+      const uint32_t back = rng() % 2 ? std::min(cb.lcup - 2, 30u) : cb.lcup - 2;
+      s[cb.lcup - 3 - rng() % back] = (uint8_t)rng();
+    }
+  }
+}
+
 int main(int argc, char** argv) {
   sgn::emu_tables();
   std::vector<int> fmts;
@@ -404,8 +425,14 @@ int main(int argc, char** argv) {
   for (int i = first; i < argc; ++i) {
     std::ifstream f(argv[i], std::ios::binary);
     std::vector<uint8_t> d((std::istreambuf_iterator<char>(f)), {});
-    if (damaged) damage_segments(d, (uint32_t)std::atoi(argv[3]) + (uint32_t)i);
-    fails += run(d, fmts) != 0;
+    if (damaged) {
+      sgn::TileLayout T;
+      sgn::parse_tile(d.data(), d.size(), nullptr, T);
+      const uint32_t seed = (uint32_t)std::atoi(argv[3]) + (uint32_t)i;
+      if (T.classic) damage_segments(d, seed);
+      else damage_cleanup(d, seed);
+    }
+    fails += run(d, fmts, damaged) != 0;
   }
   printf("fails %d\n", fails);
   return fails != 0;

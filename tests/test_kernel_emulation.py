@@ -136,3 +136,23 @@ def test_damaged_classic_segments_through_emulated_kernels(emu, style):
                                              cb_exp_h=cb_h))
     for seed in (1, 100):
         run(emu, "0", streams, ["-d", str(seed)], timeout=60)
+
+
+@pytest.mark.parametrize("seed", [10, 20, 30])
+def test_damaged_cleanup_segments_through_emulated_kernels(emu, seed):
+    """Damaged HT blocks, most of odd width, one and two per warp: where the
+    oracle decodes the damaged codestream the coefficients and pixels equal
+    its, also where the damage makes samples right of the block's last column
+    significant (which take no bits of the MagSgn stream); where it rejects the
+    codestream the kernels do so too."""
+    from signinum_b200 import encode
+    from tests.helpers import random_tile
+
+    rng = np.random.default_rng(4700)
+    streams = []
+    for w, h, bd, cb in [(65, 16, 16, 4), (63, 12, 16, 4), (33, 9, 16, 3), (31, 14, 12, 3), (9, 7, 8, 1), (129, 8, 16, 5),
+                         (7, 30, 16, 3), (13, 13, 16, 2), (65, 30, 16, 4), (67, 8, 12, 2)]:
+        px = random_tile(rng, w, h, 1, bd, 1)
+        streams.append(encode.encode_lossless(px.reshape(-1).view(np.uint8), w, h, 1, bd, levels=0, cb_exp=cb, cb_exp_h=3,
+                                              use_mct=False))
+    run(emu, "0", streams, ["-d", str(seed)])
