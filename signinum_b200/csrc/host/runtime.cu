@@ -763,10 +763,12 @@ sgn_status apply_config(sgn_ctx* ctx, sgn_plan* p, const LaunchConfig& in) {
     // Plans of at most six blocks per SM take the fused form: each block's
     // MagSgn follows its own chain instead of the slowest chain of the plan.
     // With more, the MagSgn warps take issue slots from the chains running
-    // beside them on the same SMs (one-tile plans, two kernels -> fused:
-    // 210 blocks 0.175 -> 0.138 ms, 777 blocks 0.087 -> 0.075 ms, 786
-    // 0.217 -> 0.209 ms; 1,027 blocks 0.224 -> 0.253 ms, 3,081 blocks 0.118
-    // -> 0.183 ms).
+    // beside them on the same SMs.  One-tile plans, replay of the whole plan,
+    // two kernels -> fused: 64x64 blocks 210 of them 0.162 -> 0.109 ms, 642
+    // 0.172 -> 0.154, 777 0.180 -> 0.152, 912 0.179 -> 0.182, 1,254 0.187 ->
+    // 0.219, 2,154 0.213 -> 0.287; 32x32 blocks 399 0.070 -> 0.053, 777 0.072
+    // -> 0.059, 912 0.073 -> 0.067, 1,083 0.078 -> 0.072, 1,254 0.076 ->
+    // 0.077, 1,542 0.082 -> 0.089, 2,397 0.080 -> 0.109.
     c.ht_fused = c.vlc_lanes == 1 && p->nht <= 6ull * (uint64_t)std::max(1, ctx->sm_count) &&
                          ht_magsgn_smem_bytes(p->ms_words, p->max_w, 1) <= 200 * 1024
                      ? 1

@@ -35,7 +35,7 @@ struct ResidentTile {
   std::vector<uint8_t> host;  // for header parsing
   uint64_t offset = 0;        // in the device arena (16-byte aligned)
   uint32_t width = 0, height = 0, ncomp = 0;
-  bool classic = false;  // classic (EBCOT) code blocks: per-thread scratch instead of quad symbols
+  bool classic = false;  // classic (EBCOT) code blocks: no quad symbols
   // Packet-header parse per resolution (downscale 1, 2, 4, 8), made by the
   // dispatcher the first time a request needs it and reused afterwards.
   std::unique_ptr<TileLayout> layout[4];
@@ -78,9 +78,12 @@ struct Slot {
 // Device bytes one request needs while its batch is in flight: coefficient
 // arena, level buffers and quad symbols of the decoded resolution, the output
 // surface and the job tables (about 48 bytes per code block).  Classic tiles
-// need no quad symbols but per-thread flag scratch (at most (w+2)(h+2) 16-bit
-// words per block) and, with several layers, a gathered copy of their data:
-// 3 bytes per sample covers both.
+// need no quad symbols but, in plans of more blocks than shared memory holds,
+// column words in scratch (half a byte per sample, up to two in blocks of one
+// row) and, with several layers, a gathered copy of their data: 3 bytes per
+// sample covers both.  Scratch slots have the size of the plan's largest block,
+// so a batch of thousands of small blocks beside a 64 x 64 one takes more than
+// its estimate: at most a slot for every lane of the grid, about 204 MB on a B200.
 uint64_t estimate_bytes(const ResidentTile& t, uint32_t format, const sgn_request& r) {
   const uint64_t d = (r.kind == SGN_REQ_SCALED || r.kind == SGN_REQ_REGION_SCALED) ? std::max(1u, r.downscale) : 1;
   const uint64_t w = (t.width + d - 1) / d, h = (t.height + d - 1) / d;

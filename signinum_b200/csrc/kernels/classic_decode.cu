@@ -29,16 +29,18 @@
 // the whole context window; they sit in registers while the column is coded,
 // and the next column's words are loaded one column ahead.
 //
-// What bounds it: the chain of decisions of the plan's longest block (some
-// 40,000 of them in a 64 x 64 block of noise), every decision a fixed-latency
-// path of table loads and selects in a warp that has its scheduler almost to
-// itself.  64 tiles of 512 x 512 RGB (13,440 blocks): 41.6 ms with a thread
-// per block and nested pass loops, whose 32 lanes took turns at their
-// branches (10.5 M warp instructions per warp), 21.1 ms in this form with 16
-// blocks per warp; one tile (210 blocks, one per warp) 13.7 ms, with all of
-// them in seven warps 18.3 ms.  The same loop with a branch per kind of
-// decision took 27 ms (24 ms for one tile with 16 blocks per warp).  256
-// tiles (53,760 blocks, words in scratch) 66 -> 38 ms.
+// What bounds it: the chain of decisions of the plan's longest block, every
+// iteration a fixed-latency path of table loads and selects in a warp that has
+// its scheduler almost to itself.  In one 512 x 512 RGB tile of the uniform
+// batch the longest block takes 33,302 iterations, 25,850 of them a decision
+// (the others step over a column that the pass does not code): 13.7 ms, 810
+// cycles for the 220 instructions of an iteration, with one block per warp
+// (210 of them); 18.3 ms with all of them in seven warps.  64 tiles (13,440
+// blocks): 41.6 ms with a thread per block and nested pass loops, whose 32
+// lanes took turns at their branches (10.5 M warp instructions per warp), 21.1
+// ms in this form with 16 blocks per warp.  The same loop with a branch per
+// kind of decision took 27 ms (24 ms for one tile with 16 blocks per warp).
+// 256 tiles (53,760 blocks, words in scratch) 66 -> 38 ms.
 #include <algorithm>
 #include <cstdint>
 

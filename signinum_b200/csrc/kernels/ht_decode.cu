@@ -1071,7 +1071,7 @@ __device__ void magsgn_block(const HtJob& job, const uint8_t* __restrict__ arena
   if (ok) {
     const uint32_t ms_len = lcup - scup;
     // The block's own words of the bit array (at most ms_words, checked
-    // above): they are zeroed, filled and padded with ones past the stream,
+    // above): they are written whole and padded with ones past the stream,
     // and reads beyond them return ones, so bits past the end still read as
     // the reference's 0xFF padding.
     const uint32_t words = (ms_len + 15) / 4 + 2;

@@ -1,6 +1,8 @@
 """Classic (EBCOT) plans of enough code blocks that the lanes of a warp decode
-different blocks: every lane count up to 32, blocks of partial stripes and
-columns, each style's transitions, lossless against the source pixels."""
+different blocks: 1, 8, 17 and 18 blocks per warp with the column words in
+shared memory and 32 in scratch (on 148 SMs), blocks of partial stripes and
+columns, styles' transitions, lossless against the source pixels.  Other lane
+counts, and damaged streams, run in the CPU emulation."""
 import numpy as np
 import pytest
 
@@ -8,12 +10,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("w,h,cb,cb_h,style", [
-    (64, 64, 0, 0, 0),      # 4 x 4 blocks: a few lanes of a few warps
-    (257, 131, 0, 0, 0),    # 6,500 blocks, ragged edges: eight lanes
-    (509, 303, 0, 0, 0x08),   # 29,000 blocks: 32 lanes, vertically causal
-    (509, 303, 0, 1, 0x05),   # 4 x 8, bypass and termination on every pass
-    (640, 253, 1, 0, 0x22),   # 8 x 4, context reset and segmentation symbols
-    (333, 1023, 4, 4, 0x2F),  # 64 x 64, every style at once
+    (64, 64, 0, 0, 0),      # 4 x 4, 768 blocks: one lane
+    (257, 131, 0, 0, 0),    # 6,729 blocks, ragged edges: eight lanes
+    (509, 303, 0, 0, 0x08),   # 29,280 blocks: 32 lanes, words in scratch, vertically causal
+    (509, 303, 0, 1, 0x05),   # 4 x 8, 17 lanes, bypass and termination on every pass
+    (640, 253, 1, 0, 0x22),   # 8 x 4, 18 lanes, context reset and segmentation symbols
+    (333, 1023, 4, 4, 0x2F),  # 64 x 64, one lane, every style at once
 ])
 def test_many_blocks_lossless(w, h, cb, cb_h, style):
     from signinum_b200 import encode
