@@ -593,12 +593,13 @@ __device__ __forceinline__ uint32_t ff_bytes(uint32_t x) {
 // (events, below), so that its bits are one string of n bits at bit P of the
 // stream, and writes the words of W whose first bit lies in its string, their
 // ends completed from the next lane's string by a shuffle: no word is written
-// twice but the first of a step, which lane 0 completes.  The pass is bound by
-// instruction issue: eight bytes per lane instead of four, one 64-bit load
-// instead of two unaligned words, plain stores instead of shared-memory
-// atomics into a zeroed array, and fewer operations per sample in the row
-// loops below took it from 2.70 to 2.17 ms on the uneven batch of 1,024 tiles
-// and from 0.50 to 0.41 ms on 256 tiles of 512 x 512.
+// twice but the first of a step, which lane 0 completes.  The pass issues
+// instructions in 69 % of its cycles and waits for its loads in most others:
+// eight bytes per lane instead of four, one 64-bit load instead of two
+// unaligned words, plain stores instead of shared-memory atomics into a zeroed
+// array, and fewer operations per sample in the row loops below took it from
+// 2.70 to 2.17 ms on the uneven batch of 1,024 tiles and from 0.50 to 0.41 ms
+// on 256 tiles of 512 x 512.
 template <int G>
 __device__ __forceinline__ void unstuff_magsgn(const uint8_t* src, uint32_t len, uint32_t* W, uint32_t nwords) {
   const uint32_t lane = threadIdx.x & 31, gl = lane & (G - 1), gsh = lane & (32 - G);
